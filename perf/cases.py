@@ -25,6 +25,7 @@ from ark_b200.llama import LLAMA2_7B, LLAMA2_70B, LlamaConfig, decoder_layer, la
 
 SHAPES = {"7b": LLAMA2_7B, "70b": LLAMA2_70B}
 DTYPES = {"fp32": (ark.fp32, torch.float32), "fp16": (ark.fp16, torch.float16), "bf16": (ark.bf16, torch.bfloat16)}
+STORED = {"FP32": torch.float32, "FP16": torch.float16, "BF16": torch.bfloat16, "INT32": torch.int32}
 VOCAB = 32000
 
 
@@ -124,7 +125,8 @@ def _mask(batch, seq, padded, gen):
 
 
 def _build(case, gen):
-    """Adds the case's operators to the global model: ({tensor: values}, {name: output tensor})."""
+    """Adds the case's operators to the global model: ({tensor: values}, {name: output tensor}, the inputs' tensors by
+    name: one dict for the call and one for each layer)."""
     ark.init()
     adt = DTYPES[case["dtype"]][0]
 
@@ -143,7 +145,7 @@ def _build(case, gen):
             m = _mask(batch, seq, attention == "mask", gen)
             mask = ark.tensor(list(m.shape), adt)
             feeds[mask] = m
-        h = x
+        h, named = x, [{"x": x, "rope": rope, "mask": mask}]
         for _ in range(case["layers"]):
             w = layer_weights(cfg, adt, 1)
             kc = vc = None
@@ -155,10 +157,11 @@ def _build(case, gen):
             for k, t in w.items():
                 if not (decode and k in ("wk", "wv")):  # a decode step finds its keys and values in the cache
                     feeds[t] = normal(t.shape, 0.05, 1.0) if "norm" in k else normal(t.shape, 0.02)
-        return feeds, {"hidden": h}
+            named.append({**w, "kc": kc, "vc": vc})
+        return feeds, {"hidden": h}, named
     if case["kind"] == "ffn":
         x, w1, w2, y = build_ffn(case["tokens"], case["d_model"], case["d_ff"], adt, act=case["act"], weights_nk=case["weights_nk"])
-        return {x: normal(x.shape), w1: normal(w1.shape, 0.02), w2: normal(w2.shape, 0.02)}, {"y": y}
+        return {x: normal(x.shape), w1: normal(w1.shape, 0.02), w2: normal(w2.shape, 0.02)}, {"y": y}, [{"x": x, "w1": w1, "w2": w2}]
     if case["kind"] == "rows":
         rows, cols = case["rows"], case["cols"]
         ids, table, pos = ark.tensor([rows], ark.int32), ark.tensor([VOCAB, cols], adt), ark.tensor([rows, cols], adt)
@@ -170,19 +173,19 @@ def _build(case, gen):
         pooled = ark.reduce_mean(s, axis=0)
         feeds = {ids: torch.randint(0, VOCAB, (rows,), generator=gen, device="cuda"), table: normal(table.shape), pos: normal(pos.shape, 0.1),
                  gain: normal(gain.shape, 0.05, 1.0), weight: normal(weight.shape, 0.05, 1.0)}
-        return feeds, {"stream": s, "probabilities": p, "pooled": pooled}
+        named = {"ids": ids, "table": table, "pos": pos, "gain": gain, "weight": weight}
+        return feeds, {"stream": s, "probabilities": p, "pooled": pooled}, [named]
     a, b = ark.tensor([case["rows"], case["cols"]], adt), ark.tensor([case["rows"], case["cols"]], adt)
-    return {a: normal(a.shape), b: normal(b.shape)}, {"sum": ark.add(a, b)}
+    return {a: normal(a.shape), b: normal(b.shape)}, {"sum": ark.add(a, b)}, [{"a": a, "b": b}]
 
 
 def prepare(case, seed):
     gen = torch.Generator(device="cuda").manual_seed(int(seed))
-    feeds, outs = _build(case, gen)
+    feeds, outs, _ = _build(case, gen)
     ex = ark.Executor(torch.cuda.current_device(), 0, "case", str(ark.Planner(torch.cuda.current_device()).plan()), loop_mode=False)
     ex.compile()
-    to = {"FP32": torch.float32, "FP16": torch.float16, "BF16": torch.bfloat16, "INT32": torch.int32}
     for t, values in feeds.items():
-        v = values.to(to[t.dtype.name]).contiguous()
+        v = values.to(STORED[t.dtype.name]).contiguous()
         torch.cuda.current_stream().synchronize()  # the executor copies on a stream of its own
         ex.tensor_write(t, v.data_ptr(), v.numel() * v.element_size(), is_d2d=True)
     ex.launch()
@@ -193,6 +196,70 @@ def run(state):
     state["ex"].run(1)
     state["ex"].wait()
     return state["outs"]
+
+
+def _rotate(x, table):
+    """x [batch, seq, heads, head_dim]; table [1, seq, 1, head_dim]."""
+    a, b, cos, sin = x[..., 0::2], x[..., 1::2], table[..., 0::2], table[..., 1::2]
+    return torch.stack([a * cos - b * sin, a * sin + b * cos], -1).reshape(x.shape)
+
+
+def _gelu(x):
+    return torch.nn.functional.gelu(x, approximate="tanh")
+
+
+def _rms(x, w, eps=1e-5):
+    return x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps) * w
+
+
+def _layer64(x, rope, mask, w, cfg, batch, seq, decode):
+    hd, g = cfg.head_dim, cfg.n_heads // cfg.n_kv_heads
+    h = _rms(x, w["attn_norm"], cfg.norm_eps)
+    q = _rotate((h @ w["wq"].T).view(batch, seq, cfg.n_heads, hd), rope).transpose(1, 2)
+    if decode:
+        k, v = w["kc"], w["vc"]
+    else:
+        k = _rotate((h @ w["wk"].T).view(batch, seq, cfg.n_kv_heads, hd), rope).transpose(1, 2)
+        v = (h @ w["wv"].T).view(batch, seq, cfg.n_kv_heads, hd).transpose(1, 2)
+        if mask is None:
+            mask = torch.triu(torch.full((seq, seq), -math.inf, device="cuda", dtype=torch.float64), 1)[None, None]
+    o = torch.empty_like(q)
+    for b in range(batch):
+        for n in range(cfg.n_kv_heads):  # head by head: the scores of all heads at once would take gigabytes
+            s = q[b, n * g:(n + 1) * g] @ k[b, n].T / math.sqrt(hd)
+            if mask is not None:
+                s = s + mask[min(b, mask.shape[0] - 1)]
+            o[b, n * g:(n + 1) * g] = s.softmax(-1) @ v[b, n]
+    x = x + o.transpose(1, 2).reshape(batch * seq, cfg.n_heads * hd) @ w["wo"].T
+    h = _rms(x, w["ffn_norm"], cfg.norm_eps)
+    return x + (torch.nn.functional.silu(h @ w["w1"].T) * (h @ w["w3"].T)) @ w["w2"].T
+
+
+def exact(case, seed):
+    """What run() returns for these inputs, in 64 bits throughout."""
+    feeds, outs, named = _build(case, torch.Generator(device="cuda").manual_seed(int(seed)))
+    feeds = {t: v.to(STORED[t.dtype.name]) for t, v in feeds.items()}  # the inputs as they are stored
+
+    def wide(d):
+        return {k: feeds[t].double() for k, t in d.items() if t in feeds}
+
+    g = wide(named[0])
+    if case["kind"] in ("decode", "prefill"):
+        decode, x = case["kind"] == "decode", g["x"]
+        for w in named[1:]:
+            x = _layer64(x, g["rope"], g.get("mask"), wide(w), LlamaConfig(**SHAPES[case["shape"]]), case["batch"],
+                         1 if decode else case["seq"], decode)
+        return {"hidden": x}
+    if case["kind"] == "ffn":
+        w1, w2 = (g["w1"].T, g["w2"].T) if case["weights_nk"] else (g["w1"], g["w2"])
+        act = {"relu": torch.relu, "gelu": _gelu, "silu": torch.nn.functional.silu}[case["act"]]
+        return {"y": act(g["x"] @ w1) @ w2}
+    if case["kind"] == "rows":
+        x = g["table"][g["ids"].long()] + g["pos"]
+        s = x + _gelu(torch.nn.functional.layer_norm(x, x.shape[-1:], eps=1e-5) * g["gain"])
+        p = (_rms(s, g["weight"]) / math.sqrt(128)).softmax(-1)
+        return {"stream": s, "probabilities": p, "pooled": s.mean(0, keepdim=True)}
+    return {"sum": g["a"] + g["b"]}
 
 
 def work(case):

@@ -747,75 +747,4 @@ __device__ __noinline__ void run_splitk_reduce(const SplitKReduceArgs &a, int p,
     else splitk_reduce_typed<__half>(a, p, P);
 }
 
-// ---- CUDA-core fallback -------------------------------------------------------------
-// For operands the TMA path cannot describe (row pitch or base not 16-byte
-// aligned) and for fp32. 64x64 tile per CTA pass, fp32 accumulate.
-template <typename T>
-__device__ void gemm_simt_typed(const GemmSimtArgs &g, int p, int P, char *smem) {
-    constexpr int TM = 64, TN = 64, TK = 16;
-    float(*sA)[TM + 1] = reinterpret_cast<float(*)[TM + 1]>(smem);                          // [TK][TM+1]
-    float(*sB)[TN + 1] = reinterpret_cast<float(*)[TN + 1]>(smem + TK * (TM + 1) * 4);      // [TK][TN+1]
-    const int tiles_m = (g.M + TM - 1) / TM, tiles_n = (g.N + TN - 1) / TN;
-    const int per = tiles_m * tiles_n;
-    const int total = per * g.batch_c * g.batch_n;
-    const int tid = threadIdx.x;
-    // 512 threads: thread computes a 2x4 block of the 64x64 tile
-    const int ty = tid / 16, tx = tid % 16;  // ty 0..31 -> rows ty*2.., tx -> cols tx*4..
-    for (int u = p; u < total; u += P) {
-        const int b = u / per, r = u % per;
-        const int bc = b % g.batch_c, bn = b / g.batch_c;
-        const int m0 = (r / tiles_n) * TM, n0 = (r % tiles_n) * TN;
-        const T *A = reinterpret_cast<const T *>(g.A) + bn * g.a_stride_n + bc * g.a_stride_c;
-        const T *B = reinterpret_cast<const T *>(g.B) + bn * g.b_stride_n + bc * g.b_stride_c;
-        T *C = reinterpret_cast<T *>(g.C) + bn * g.c_stride_n + bc * g.c_stride_c;
-        float acc[2][4] = {};
-        for (int k0 = 0; k0 < g.K; k0 += TK) {
-            for (int i = tid; i < TK * TM; i += kThreads) {
-                int kk = i / TM, mm = i % TM;
-                if (!g.trans_a) { mm = i / TK; kk = i % TK; }
-                int m = m0 + mm, k = k0 + kk;
-                float v = 0.0f;
-                if (m < g.M && k < g.K) v = to_f32(g.trans_a ? A[(int64_t)k * g.lda + m] : A[(int64_t)m * g.lda + k]);
-                sA[kk][mm] = v;
-            }
-            for (int i = tid; i < TK * TN; i += kThreads) {
-                int kk = i / TN, nn = i % TN;
-                if (g.trans_b) { nn = i / TK; kk = i % TK; }
-                int n = n0 + nn, k = k0 + kk;
-                float v = 0.0f;
-                if (n < g.N && k < g.K) v = to_f32(g.trans_b ? B[(int64_t)n * g.ldb + k] : B[(int64_t)k * g.ldb + n]);
-                sB[kk][nn] = v;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int kk = 0; kk < TK; ++kk) {
-                float a0 = sA[kk][ty * 2], a1 = sA[kk][ty * 2 + 1];
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    float bv = sB[kk][tx * 4 + j];
-                    acc[0][j] += a0 * bv;
-                    acc[1][j] += a1 * bv;
-                }
-            }
-            __syncthreads();
-        }
-#pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                int m = m0 + ty * 2 + i, n = n0 + tx * 4 + j;
-                if (m < g.M && n < g.N) C[(int64_t)m * g.ldc + n] = from_f32<T>(apply_act(g.act, acc[i][j]));
-            }
-    }
-}
-
-__device__ __noinline__ void run_gemm_simt(const GemmSimtArgs &g, int p, int P, char *smem) {
-    switch (g.dtype) {
-        case DT_F32: gemm_simt_typed<float>(g, p, P, smem); break;
-        case DT_F16: gemm_simt_typed<__half>(g, p, P, smem); break;
-        case DT_BF16: gemm_simt_typed<__nv_bfloat16>(g, p, P, smem); break;
-        default: break;
-    }
-}
-
 }  // namespace arkb

@@ -668,6 +668,41 @@ struct Lowerer {
                (bst[3] * es) % 16 == 0 && (ast[2] * ast[3] * es) % 16 == 0 && (bst[2] * bst[3] * es) % 16 == 0;
     }
 
+    // ---- the CUDA-core matmul's tile and split ------------------------------------------------
+    static constexpr int64_t kSimtTileElems = 64 * 256;  // the same for all three tiles
+    static int64_t simt_tiles(const GemmSimtArgs &g) {
+        const int64_t tm = 32 * g.wm, tn = 512 / g.wm;
+        return (g.M + tm - 1) / tm * ((g.N + tn - 1) / tn) * g.batch_c * g.batch_n;
+    }
+    static void split_simt(GemmSimtArgs &g, int64_t P) {
+        // The tile with the least padding; flat tiles move more operand bytes per multiply-add, so they are for few rows.
+        const double cost[3] = {1.0, 1.05, 1.3};
+        double best = 1e300;
+        for (int i = 0, wm = 4; i < 3; ++i, wm /= 2) {
+            GemmSimtArgs t = g;
+            t.wm = wm;
+            const double c = (double)simt_tiles(t) * cost[i];
+            if (c < best * 0.999) { best = c; g.wm = wm; }
+        }
+        const int64_t tk = g.wm == 1 ? 8 : 16;
+        g.kblocks = (int32_t)std::max<int64_t>(1, (g.K + tk - 1) / tk);
+        const int64_t tiles = simt_tiles(g), n = tiles * g.kblocks;
+        // Equal runs over all CTAs, a barrier and a sum of the shared tiles, against a tile per CTA: the sum and its
+        // barrier take about as long as 10 k-blocks of 16, so short or well-filled problems are not cut.
+        const int64_t sum_cost = 10 * 16 / tk, runs = std::min(P, (n + 7) / 8);
+        const int64_t even = (n + runs - 1) / runs + sum_cost, whole = (tiles + P - 1) / P * g.kblocks;
+        if (whole <= even && (tiles <= P || tiles % P == 0)) g.runs = (int32_t)std::min(tiles, P);
+        else g.runs = (int32_t)runs;
+        g.run_len = (int32_t)(n / g.runs);
+        g.run_rem = (int32_t)(n % g.runs);
+        const size_t es = dtype_size(g.dtype);
+        auto vec = [&](const void *p, int64_t ld, int64_t sc, int64_t sn) {
+            return reinterpret_cast<uintptr_t>(p) % (4 * es) == 0 && ld % 4 == 0 && sc % 4 == 0 && sn % 4 == 0 ? 1 : 0;
+        };
+        g.vec_a = vec(g.A, g.lda, g.a_stride_c, g.a_stride_n);
+        g.vec_b = vec(g.B, g.ldb, g.b_stride_c, g.b_stride_n);
+    }
+
     void lower_matmul(const OpDesc &op, const Range &proc, const TaskGroup &tg, int act, const TensorDesc *act_out,
                       const OpDesc *fuse_ar = nullptr, const GemvFuse *gf = nullptr, const TensorDesc *epi = nullptr,
                       int epi_mode = 0 /* 0: add, 1: multiply, 2: rotary table [rope_rows][rope_cols] */, int64_t rope_rows = 0,
@@ -719,7 +754,29 @@ struct Lowerer {
             g.batch_c = (int32_t)bc; g.batch_n = (int32_t)bn;
             g.trans_a = ta; g.trans_b = tb;
             g.dtype = A.dtype; g.act = act;
-            push(s, "Matmul(simt) " + op.name + " M=" + std::to_string(M) + " N=" + std::to_string(N) + " K=" + std::to_string(K));
+            split_simt(g, proc.count());
+            const bool shared = g.kblocks > 1 && simt_tiles(g) % g.runs != 0;
+            const size_t ws_bytes = shared ? (size_t)g.runs * 2 * kSimtTileElems * sizeof(float) : 0;
+            if (shared) {
+                g.ws = reinterpret_cast<float *>(env.workspace + prog.workspace_bytes);
+                prog.workspace_bytes += ws_bytes;
+                acc_begin();
+                rd(A); rd_streamed(B); wr_raw(g.ws, ws_bytes);
+                if (simt_tiles(g) > 1) wr(C);  // the tiles that one run holds
+            }
+            push(s, "Matmul(simt) " + op.name + " M=" + std::to_string(M) + " N=" + std::to_string(N) + " K=" + std::to_string(K) + " tile=" +
+                        std::to_string(32 * g.wm) + "x" + std::to_string(512 / g.wm) + " runs=" + std::to_string(g.runs));
+            if (shared) {
+                GemmSimtArgs sum = g;
+                emit_sync(proc);
+                Stage r = new_stage(SK_GEMM_SIMT, proc);
+                r.gs = sum;
+                r.gs.phase = 1;
+                acc_begin();
+                rd_raw(sum.ws, ws_bytes);
+                wr(C);
+                push(r, "  sum of shared tiles " + op.name);
+            }
             return;
         }
         // One or two rows of activations against an unbatched weight matrix: the work is a read of the weights at
@@ -2440,7 +2497,11 @@ struct Lowerer {
             switch (s.kind) {
                 case SK_GEMM: need = kFullSmemBytes; break;
                 case SK_PREFILL_ATTN: need = kFullSmemBytes; break;
-                case SK_GEMM_SIMT: need = 16 * 1024; break;
+                case SK_GEMM_SIMT: {  // two buffers of k-blocks of both operands for each group of threads, every k padded by 4 floats
+                    const size_t tk = s.gs.wm == 1 ? 8 : 16;
+                    need = 4 * tk * (size_t)(32 * s.gs.wm + 4 + 512 / s.gs.wm + 4) * sizeof(float) + 1024;
+                    break;
+                }
                 case SK_REDUCE: need = (size_t)kThreads * 8 * sizeof(float); break;
                 case SK_ROWOP:
                     if (s.ro.staged_warps > 0) {

@@ -96,6 +96,33 @@ def test_matmul_cuda_core_fallback(dt, mnk):
         assert_matmul_close(got, want, dt, "simt fp16")
 
 
+@pytest.mark.parametrize("dt,ash,bsh,ta,tb", [
+    ("fp32", (1, 1), (1, 1), False, False),                     # one k-block, one tile
+    ("fp32", (16, 17), (17, 513), False, False),                # 16-row tiles, one column over, odd k
+    ("fp32", (33, 2048), (2048, 100), False, False),            # few tiles: every run holds a piece
+    ("fp32", (300, 1024), (4096, 1024), False, True),           # tiles shared between neighbouring runs
+    ("fp32", (1000, 96), (200, 1000), True, True),              # unsplit and split remainders, A transposed
+    ("fp32", (2, 3, 65, 129), (1, 3, 129, 130), False, False),  # batches with a broadcast operand
+    ("fp32", (148, 64, 40), (40, 128), False, False),           # as many tiles as processors
+    ("bf16", (31, 1001), (1001, 259), False, False),
+    ("fp16", (70, 333), (129, 333), False, True),
+])
+def test_matmul_cuda_core_tiles_and_runs(dt, ash, bsh, ta, tb):
+    """Edges of the CUDA-core form's three tiles and of its split of the k-blocks over the processors."""
+    rng = np.random.default_rng(35)
+    a, b = rand(rng, ash, dt), rand(rng, bsh, dt)
+    ark.init()
+    t_a, t_b = ark.tensor(list(ash), NAME[dt]), ark.tensor(list(bsh), NAME[dt])
+    out = ark.matmul(t_a, t_b, transpose_input=ta, transpose_other=tb)
+    (got,) = execute([out], {t_a: a, t_b: b})
+    f = lambda v, t: np.swapaxes(O.to_f32(v, dt).astype(np.float64), -1, -2) if t else O.to_f32(v, dt).astype(np.float64)
+    a64, b64 = f(a, ta), f(b, tb)
+    want = a64 @ b64
+    # k products summed in fp32 in some order, then one rounding to the storage type
+    bound = (a64.shape[-1] + 2) * 2.0 ** -24 * (np.abs(a64) @ np.abs(b64)) + {"fp32": 0, "fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want)
+    assert (np.abs(O.to_f32(got, dt) - want) <= bound + 1e-30).all()
+
+
 def test_matmul_partial_task_range_follows_plan_tiles():
     """A hand-written plan that splits one Matmul's tiles over two processor groups
     (as examples/tutorial/plan_tutorial.py does) must compute the same result."""

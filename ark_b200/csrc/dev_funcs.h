@@ -10,6 +10,7 @@ __device__ void run_ewise(const EwiseArgs &a, int p, int P, unsigned long long i
 __device__ void run_reduce(const ReduceArgs &a, int p, int P, char *smem);
 __device__ void run_rowop(const RowOpArgs &a, int p, int P, char *smem, CtaCtl *ctl, DeviceState *st, int stage_idx,
                           unsigned long long wait_limit);
+__device__ void run_rowchain(const RowChainArgs &a, int p, int P);
 __device__ void run_transpose(const TransposeArgs &a, int p, int P, char *smem);
 __device__ void run_embed(const EmbedArgs &a, int p, int P);
 // `g` may be a copy of the stage record in shared memory; `gmaps` is the record in global memory (tensor maps are read there)

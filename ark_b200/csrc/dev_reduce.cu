@@ -147,9 +147,11 @@ __device__ void reduce_other_axis(const ReduceArgs &a, int p, int P, float *red)
     const int64_t astr = a.in.stride[ax];
     const int op = a.op;
     // With fewer output vectors than threads, S threads of a CTA share one output vector: each walks 1/S of the
-    // reduced axis and the partial results are added through shared memory (segment order: deterministic).
+    // reduced axis and the partial results are added through shared memory (a fixed tree: deterministic). Up to 128
+    // segments, so that 4 neighbouring vectors (64 bytes of a row) are the least a CTA takes: 8192 rows of 4096 bf16 are
+    // 512 vectors, which 16 segments left to 16 CTAs (90 us), 128 spread over 128 (@@RED@@).
     int S = 1;
-    while (S < 16 && units * S * 2 <= (int64_t)P * kThreads && len / (S * 2) >= 16) S *= 2;
+    while (S < 128 && units * S * 2 <= (int64_t)P * kThreads && len / (S * 2) >= 16) S *= 2;
     const int UPB = kThreads / S;  // output vectors per CTA pass
     const int ul = threadIdx.x % UPB, seg = threadIdx.x / UPB;
     const int64_t k_lo = len * seg / S, k_hi = len * (seg + 1) / S;
@@ -186,16 +188,17 @@ __device__ void reduce_other_axis(const ReduceArgs &a, int p, int P, float *red)
         }
         if (S > 1) {
             __syncthreads();  // the previous pass no longer reads `red`
-            if (seg > 0) {
+            for (int half = S / 2; half > 0; half /= 2) {
+                // the upper half of the segments hand their results to the lower half
+                if (seg >= half && seg < 2 * half) {
 #pragma unroll
-                for (int i = 0; i < V; ++i) red[((size_t)seg * UPB + ul) * V + i] = acc[i];
-            }
-            __syncthreads();
-            if (seg == 0) {
-                for (int sg = 1; sg < S; ++sg) {
+                    for (int i = 0; i < V; ++i) red[((size_t)seg * UPB + ul) * V + i] = acc[i];
+                }
+                __syncthreads();
+                if (seg < half) {
 #pragma unroll
                     for (int i = 0; i < V; ++i) {
-                        const float x = red[((size_t)sg * UPB + ul) * V + i];
+                        const float x = red[((size_t)(seg + half) * UPB + ul) * V + i];
                         acc[i] = (op == RD_MAX) ? fmaxf(acc[i], x) : acc[i] + x;
                     }
                 }

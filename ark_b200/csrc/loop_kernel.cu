@@ -59,6 +59,7 @@ __device__ __forceinline__ void run_body(const LaunchParams &P, char *smem, Gemm
         cur ^= 1;
         int p = 0, Pn = 1;
         if (!in_range(S, cta, p, Pn)) continue;
+        if (S.work > 0 && p >= S.work) continue;
         if (ctl->abort) return;
         unsigned long long *stamp = P.stage_times ? P.stage_times + ((size_t)s * gridDim.x + cta) * 2 : nullptr;
         if (stamp && threadIdx.x == 0) stamp[0] = globaltimer();
@@ -84,6 +85,7 @@ __device__ __forceinline__ void run_body(const LaunchParams &P, char *smem, Gemm
             case SK_EWISE: run_ewise(S.ew, p, Pn, iter_no); break;
             case SK_REDUCE: run_reduce(S.rd, p, Pn, smem); break;
             case SK_ROWOP: run_rowop(S.ro, p, Pn, smem, ctl, P.state, s, P.spin_limit); break;
+            case SK_ROWCHAIN: run_rowchain(S.rc, p, Pn); break;
             case SK_GEMM:
                 if constexpr (PAIR) run_gemm_pair(S.gm, &P.stages[s].gm, p, Pn, smem, pipe, ctl, P.state, s, P.spin_limit);
                 else run_gemm(S.gm, &P.stages[s].gm, p, Pn, smem, pipe, ctl, P.state, s, P.spin_limit);

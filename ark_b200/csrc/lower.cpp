@@ -482,6 +482,8 @@ struct Lowerer {
                 a.staged_warps = (int32_t)std::min<int64_t>(16, total / a.staged_bufs);
             }
         }
+        if (a.warps_per_row && !a.staged_warps)
+            s.work = (int32_t)std::min<int64_t>(proc.count(), std::max<int64_t>(1, (a.rows * a.warps_per_row + kThreads / 32 - 1) / (kThreads / 32)));
         push(s, op.type + " " + op.name + " rows=" + std::to_string(a.rows) + " cols=" + std::to_string(a.cols) +
                     " warps/row=" + std::to_string(a.warps_per_row) +
                     (a.staged_warps ? " staged(" + std::to_string(a.staged_warps) + " warps x " + std::to_string(a.staged_bufs) + " rows)" : "") + part_note);
@@ -1263,6 +1265,7 @@ struct Lowerer {
         if (g.splits > 1) wr_raw(g.ws, (size_t)g.splits * bn * bc * M * N * sizeof(float));
         else wr(C);
         if (fuse_ar) acc.opaque = true;  // tiles go to the peers' staging slots
+        s.work = (int32_t)std::min<int64_t>(proc.count(), (prog.pair_mode ? 2 : 1) * std::max<int64_t>(1, g.n_units));
         push(s, std::string("Matmul ") + op.name + " M=" + std::to_string(M) + " N=" + std::to_string(N) + " K=" +
                     std::to_string(K) + " tile_n=" + std::to_string(g.tile_n) + " units=" + std::to_string(g.n_units) +
                     (g.tall ? " tall" : "") + (g.plan_tiles ? " plan-tiles" : "") + (g.act ? " act=" + std::to_string(g.act) : "") +
@@ -1356,6 +1359,7 @@ struct Lowerer {
         if (rope) { rd(rope->reads[0]); rd(rope->reads[1]); } else rd(q);
         rd_streamed(k); rd_streamed(v);
         wr_raw(a.ws, bytes);
+        s.work = (int32_t)std::min<int64_t>(P, B * Hkv * chunks);
         push(s, "DecodeAttention " + op.name + " B=" + std::to_string(B) + " heads=" + std::to_string(Hq) + "/" + std::to_string(Hkv) +
                     " keys=" + std::to_string(T) + " chunks=" + std::to_string(chunks) + " x " + std::to_string(chunk_len) + (rope ? " <-rope" : ""));
         // When the only reader of the result is the weight-streaming matmul of the next processor group (one or two
@@ -1376,6 +1380,7 @@ struct Lowerer {
         }
         emit_sync(proc);
         Stage m = s;
+        m.work = 0;
         m.da.phase = 1;
         acc_begin();
         rd_raw(a.ws, bytes);
@@ -2264,6 +2269,273 @@ struct Lowerer {
         prog = out;
     }
 
+    // ---- row chains -----------------------------------------------------------------------------------
+    // Stages that follow each other over the whole grid with nothing but a barrier in between, each working row by row
+    // on the dense result of the one before, become one SK_ROWCHAIN stage. All results are stored as before; operands
+    // of the chain and its results must either not overlap or be the same elements (every element is then read and
+    // written by one thread, in the operators' order).
+    struct Chain {
+        RowChainArgs a;
+        int64_t nelem = 0, cols = 0;
+        bool whole_rows = false;
+        int dtype = -1, esize = 0;
+        const void *cur = nullptr;                                  // the value the next operator has to work on
+        std::vector<std::pair<uintptr_t, uintptr_t>> own, outs, foreign;  // read element by element; written; read otherwise
+        std::vector<const void *> norm_in;                          // per op: what a norm without residual reads, else null
+        int stages = 0;
+    };
+    bool whole_grid(const Stage &s) const { return s.proc_b == 0 && s.proc_s == 1 && s.proc_e == prog.grid; }
+    static bool clash(const std::vector<std::pair<uintptr_t, uintptr_t>> &v, const std::pair<uintptr_t, uintptr_t> &a, bool same_ok) {
+        for (auto &e : v)
+            if (overlap(e, a) && !(same_ok && e == a)) return true;
+        return false;
+    }
+    static bool chain_reads(Chain &c, const void *p, int64_t elems) {  // element by element
+        const auto sp = span_of(p, (size_t)elems * c.esize);
+        if (!aligned16(p) || clash(c.outs, sp, true)) return false;
+        c.own.push_back(sp);
+        return true;
+    }
+    static bool chain_reads_all(Chain &c, const void *p, size_t bytes, bool vec = true) {  // by every row
+        const auto sp = span_of(p, bytes);
+        if ((vec && !aligned16(p)) || clash(c.outs, sp, false)) return false;
+        c.foreign.push_back(sp);
+        return true;
+    }
+    static bool chain_writes(Chain &c, const void *p, size_t bytes) {
+        const auto sp = span_of(p, bytes);
+        if (!aligned16(p) || clash(c.own, sp, true) || clash(c.outs, sp, true) || clash(c.foreign, sp, false)) return false;
+        c.outs.push_back(sp);
+        return true;
+    }
+    static bool chain_type(Chain &c, int dt) {
+        if (!fp_type(dt) || (c.dtype >= 0 && c.dtype != dt) || (c.esize && c.esize != (int)dtype_size(dt))) return false;
+        c.dtype = dt;
+        c.esize = (int)dtype_size(dt);
+        return true;
+    }
+    static bool chain_cols(Chain &c, int64_t cols) {
+        if (cols <= 0 || (c.cols && c.cols != cols)) return false;
+        c.cols = cols;
+        return true;
+    }
+    // Splits rows over warps; false when a row does not fit the registers of a CTA.
+    bool chain_split(Chain &c) const {
+        const int64_t V = 16 / c.esize, P = prog.grid, warps = kThreads / 32;
+        if (c.cols <= 0 || c.cols % V || c.nelem % c.cols || c.nelem / c.cols > INT32_MAX) return false;
+        const int64_t nv = c.cols / V, rows = c.nelem / c.cols;
+        if (nv < 24 && rows > warps * P) return false;  // most lanes would idle through many rows
+        int64_t segs = 1, g = 0;
+        if (!c.whole_rows)
+            for (int64_t n = 1; n <= nv && !g; ++n)  // segments of one warp, down to one vector per lane while warps are idle
+                if (nv % n == 0 && nv / n <= 32 * 4 && (rows * n >= warps * P || nv / n <= 32)) { segs = n; g = 1; }
+        if (!g) {
+            for (g = 1; g <= warps && nv > 32 * 4 * g; g *= 2) {}  // 4 vectors per lane leave room for a second operand
+            if (g > warps) g = warps;
+            if (nv > 32 * 8 * g) return false;
+            while (g < warps && rows * g < warps * P && nv > 32 * g) g *= 2;
+        }
+        c.a.warps = (int32_t)g;
+        c.a.segs = (int32_t)segs;
+        c.a.rows = (int32_t)rows;
+        c.a.cols = (int32_t)(c.cols / segs);
+        return true;
+    }
+    // Adds stage `s` to the chain; false (and the chain is not to be used) when it does not belong there.
+    bool chain_add(Chain &c, const Stage &s) const {
+        const bool first = c.stages == 0;
+        ++c.stages;
+        if (s.kind == SK_EMBED) {
+            const EmbedArgs &e = s.em;
+            if (!first || e.task_b != 0 || e.task_s != 1 || e.out_ld != e.emb_dim || e.n_idx <= 0 || e.w_ld * e.esize % 16) return false;
+            c.esize = e.esize;
+            c.nelem = e.n_idx * e.emb_dim;
+            c.a.head = RH_GATHER;
+            c.a.src = e.weight; c.a.idx = e.idx; c.a.src_ld = e.w_ld; c.a.num_emb = e.num_emb; c.a.out = e.out;
+            c.cur = e.out;
+            return chain_cols(c, e.emb_dim) && chain_reads_all(c, e.weight, (size_t)(e.num_emb * e.w_ld) * e.esize) &&
+                   chain_reads_all(c, e.idx, (size_t)e.n_idx * 4, false) && chain_writes(c, e.out, (size_t)c.nelem * c.esize);
+        }
+        if (s.kind == SK_SPLITK_REDUCE) {
+            const SplitKReduceArgs &r = s.sr;
+            if (!first || r.batch_c != 1 || r.batch_n != 1 || r.ldc != r.N || !chain_type(c, r.dtype) || !aligned16(r.ws)) return false;
+            c.nelem = (int64_t)r.M * r.N;
+            c.a.head = RH_SUM;
+            c.a.ws = r.ws; c.a.splits = r.splits; c.a.add = r.bias; c.a.act = r.act; c.a.out = r.C;
+            c.cur = r.C;
+            return chain_cols(c, r.N) && (!r.bias || chain_reads(c, r.bias, c.nelem)) && chain_writes(c, r.C, (size_t)c.nelem * c.esize);
+        }
+        if (c.a.n_ops >= kMaxChainOps || (c.a.n_ops && c.a.ops[c.a.n_ops - 1].kind == RC_CAST)) return false;
+        RowChainOp &o = c.a.ops[c.a.n_ops++];
+        std::memset(&o, 0, sizeof(o));
+        c.norm_in.push_back(nullptr);
+        if (s.kind == SK_ROWOP) {
+            const RowOpArgs &r = s.ro;
+            if (r.mask || r.in_ld != r.cols || r.out_ld != r.cols || r.rows <= 0 || !chain_type(c, r.dtype) || !chain_cols(c, r.cols)) return false;
+            if (first) { c.nelem = r.rows * r.cols; c.cur = r.in; c.a.src = r.in; if (!chain_reads(c, r.in, c.nelem)) return false; }
+            if (c.nelem != r.rows * r.cols) return false;
+            c.whole_rows = true;
+            o.kind = r.op == RO_RMSNORM ? RC_RMSNORM : r.op == RO_LAYERNORM ? RC_LAYERNORM : RC_SOFTMAX;
+            o.scalar = o.kind == RC_SOFTMAX ? r.scale : r.eps;
+            if (r.residual) {
+                if (o.kind != RC_RMSNORM || r.in == r.residual || (c.cur != r.in && c.cur != r.residual)) return false;
+                o.other_mode = 1;
+                o.other = c.cur == r.in ? r.residual : r.in;
+                o.out2 = r.res_out;
+                if (!chain_reads(c, o.other, c.nelem) || !chain_writes(c, r.res_out, (size_t)c.nelem * c.esize)) return false;
+            } else {
+                if (c.cur != r.in) return false;
+                c.norm_in.back() = r.in;
+            }
+            if (r.weight) {
+                o.weight = r.weight;
+                o.weight_f32 = r.weight_f32;
+                if (!chain_reads_all(c, r.weight, (size_t)r.cols * (r.weight_f32 ? 4 : c.esize))) return false;
+            }
+            o.out = r.out;
+            c.cur = r.out;
+            return chain_writes(c, r.out, (size_t)c.nelem * c.esize) && chain_split(c);
+        }
+        if (s.kind != SK_EWISE) return false;
+        const EwiseArgs &e = s.ew;
+        if (e.iter_slots > 1 || e.task_s != 0 || e.vec <= 1 || e.op == EW_COPY || e.op == EW_ROPE || e.op == EW_SCALAR_ASSIGN) return false;
+        const bool binary = e.op >= EW_ADD && e.op <= EW_DIV;
+        int64_t n;
+        if (e.flat) {
+            n = e.n_units * e.vec;
+        } else {  // [rows, cols] after the collapse of dimensions
+            if (e.out.shape[0] != 1 || e.out.shape[1] != 1 || e.out.stride[3] != 1 || e.out.stride[2] != e.out.shape[3]) return false;
+            n = (int64_t)e.out.shape[2] * e.out.shape[3];
+            if (!chain_cols(c, e.out.shape[3])) return false;
+        }
+        // 0: tensor, 1: one row for all rows, -1: neither
+        auto form = [&](const TRef &t) {
+            if (e.flat) return 0;
+            if (t.stride[3] != 1) return -1;
+            return t.stride[2] == t.shape[3] ? 0 : t.stride[2] == 0 ? 1 : -1;
+        };
+        const int f0 = form(e.in0), f1 = binary ? form(e.in1) : -1;
+        if (e.op == EW_CAST) {
+            if (!e.flat || first || e.out.dtype == e.in0.dtype || !fp_type(e.out.dtype) || !chain_type(c, e.in0.dtype) || c.cur != e.in0.ptr || n != c.nelem)
+                return false;
+            o.kind = RC_CAST;
+            o.op = e.out.dtype;
+            o.out = e.out.ptr;
+            c.cur = nullptr;
+            return chain_writes(c, o.out, (size_t)n * dtype_size(e.out.dtype));
+        }
+        if (e.out.dtype != e.in0.dtype || (binary && e.in1.dtype != e.in0.dtype) || !chain_type(c, e.out.dtype)) return false;
+        if (first) {
+            c.nelem = n;
+            const TRef &t = f0 == 0 ? e.in0 : e.in1;
+            if (f0 != 0 && (!binary || f1 != 0)) return false;
+            c.cur = t.ptr;
+            c.a.src = t.ptr;
+            if (!chain_reads(c, t.ptr, n)) return false;
+        }
+        if (n != c.nelem) return false;
+        o.kind = RC_EWISE;
+        o.op = e.op;
+        o.scalar = e.scalar;
+        const bool cur0 = f0 == 0 && e.in0.ptr == c.cur, cur1 = f1 == 0 && e.in1.ptr == c.cur;
+        if (!cur0 && !cur1) return false;
+        if (cur0 && cur1) o.other_mode = 3;
+        else if (binary) {
+            const int f = cur0 ? f1 : f0;
+            const TRef &t = cur0 ? e.in1 : e.in0;
+            if (f < 0) return false;
+            o.other_mode = f == 0 ? 1 : 2;
+            o.other = t.ptr;
+            o.swapped = cur0 ? 0 : 1;
+            if (!(f == 0 ? chain_reads(c, t.ptr, n) : chain_reads_all(c, t.ptr, (size_t)t.shape[3] * c.esize))) return false;
+        }
+        o.out = e.out.ptr;
+        c.cur = e.out.ptr;
+        return chain_writes(c, o.out, (size_t)n * c.esize);
+    }
+    // A later stage that is the same norm of the same rows as an operator of the chain, with nothing in between that
+    // changes its operands or touches its result: the chain stores the result there too. Returns its index or 0.
+    size_t equal_norm(const Chain &c, size_t k, size_t after) const {
+        const RowChainOp &o = c.a.ops[k];
+        if (!c.norm_in[k] || o.kind == RC_SOFTMAX) return 0;
+        const auto in = span_of(c.norm_in[k], (size_t)c.nelem * c.esize), w = span_of(o.weight, (size_t)c.cols * (o.weight_f32 ? 4 : c.esize));
+        auto is_same = [&](const Stage &s) {
+            const RowOpArgs &r = s.ro;
+            return s.kind == SK_ROWOP && whole_grid(s) && !r.mask && !r.residual && r.in == c.norm_in[k] && r.weight == o.weight && r.eps == o.scalar &&
+                   (r.op == RO_RMSNORM ? RC_RMSNORM : r.op == RO_LAYERNORM ? RC_LAYERNORM : RC_SOFTMAX) == o.kind && r.dtype == c.dtype &&
+                   r.weight_f32 == o.weight_f32 && r.cols == c.cols && r.in_ld == r.cols && r.out_ld == r.cols && r.rows * r.cols == c.nelem && aligned16(r.out);
+        };
+        for (size_t j = after; j < prog.stages.size() && j < after + 12; ++j) {
+            const StageAccess &x = prog.access[j];
+            if (is_same(prog.stages[j])) {
+                const auto out = span_of(prog.stages[j].ro.out, (size_t)c.nelem * c.esize);
+                if (clash(c.own, out, false) || clash(c.outs, out, false) || clash(c.foreign, out, false)) return 0;
+                for (size_t m = after; m < j; ++m)
+                    if (clash(prog.access[m].reads, out, false) || clash(prog.access[m].writes, out, false)) return 0;
+                return j;
+            }
+            if (prog.stages[j].kind != SK_SYNC && (x.opaque || clash(x.writes, in, false) || (o.weight && clash(x.writes, w, false)))) return 0;
+        }
+        return 0;
+    }
+    void fuse_row_chains() {
+        if (const char *e = getenv("ARKB_KEEP_SYNCS")) if (atoi(e)) return;
+        auto erase = [&](size_t b, size_t e) {
+            prog.stages.erase(prog.stages.begin() + b, prog.stages.begin() + e);
+            prog.access.erase(prog.access.begin() + b, prog.access.begin() + e);
+            prog.notes.erase(prog.notes.begin() + b, prog.notes.begin() + e);
+        };
+        for (size_t i = 0; i < prog.stages.size(); ++i) {
+            // the barrier in front also orders what the later members depend on
+            if (i > 0 && !(prog.stages[i - 1].kind == SK_SYNC && whole_grid(prog.stages[i - 1]))) continue;
+            Chain c;
+            std::memset(&c.a, 0, sizeof(c.a));
+            if (!whole_grid(prog.stages[i]) || prog.access[i].opaque || !chain_add(c, prog.stages[i])) continue;
+            size_t last = i;
+            Chain best;
+            std::memset(&best.a, 0, sizeof(best.a));
+            while (last + 2 < prog.stages.size() && prog.stages[last + 1].kind == SK_SYNC && whole_grid(prog.stages[last + 1]) &&
+                   whole_grid(prog.stages[last + 2]) && !prog.access[last + 2].opaque) {
+                Chain t = c;
+                if (!chain_add(t, prog.stages[last + 2])) break;
+                c = t;
+                last += 2;
+                if (chain_split(c)) best = c;  // (without a row width yet, or with rows that do not fit, it cannot end here)
+            }
+            if (best.stages < 2) continue;
+            last = i + 2 * (size_t)(best.stages - 1);
+            Stage s = new_stage(SK_ROWCHAIN, Range{0, prog.grid, 1});
+            best.a.dtype = best.dtype;
+            StageAccess x;
+            x.opaque = false;
+            std::string note = "[0," + std::to_string(prog.grid) + ") Row chain rows=" + std::to_string(best.a.rows) + " cols=" + std::to_string(best.cols) +
+                               (best.a.segs > 1 ? " segments=" + std::to_string(best.a.segs) : "") + " warps=" + std::to_string(best.a.warps) + ":";
+            for (size_t j = i; j <= last; j += 2) {
+                const StageAccess &y = prog.access[j];
+                x.reads.insert(x.reads.end(), y.reads.begin(), y.reads.end());
+                x.writes.insert(x.writes.end(), y.writes.begin(), y.writes.end());
+                x.streamed.insert(x.streamed.end(), y.streamed.begin(), y.streamed.end());
+                const std::string &nt = prog.notes[j];
+                const size_t b = nt.find_first_not_of(' ', nt.find(") ") + 2), at = nt.find(' ', b);  // the operator's type
+                note += std::string(j > i ? ", " : " ") + nt.substr(b, at - b);
+            }
+            for (size_t k = 0; k < (size_t)best.a.n_ops; ++k)
+                if (const size_t j = equal_norm(best, k, last + 1)) {
+                    best.a.ops[k].copy = prog.stages[j].ro.out;
+                    best.outs.push_back(span_of(best.a.ops[k].copy, (size_t)best.nelem * best.esize));
+                    x.writes.push_back(best.outs.back());
+                    note += " (+ " + prog.notes[j].substr(prog.notes[j].find(") ") + 2, prog.notes[j].find(" rows=") - prog.notes[j].find(") ") - 2) + ")";
+                    erase(j, j + 1);
+                }
+            s.rc = best.a;
+            s.work = (int32_t)std::min<int64_t>(prog.grid, ((int64_t)best.a.rows * best.a.segs * best.a.warps + kThreads / 32 - 1) / (kThreads / 32));
+            prog.stages[i] = s;
+            prog.access[i] = x;
+            prog.notes[i] = note;
+            erase(i + 1, last + 1);
+        }
+    }
+
     // Two weight-streaming matmuls that follow each other without a barrier, over the same activations with the same
     // prologue and of the same shape (W1 and W3 of a SwiGLU block), become one stage: x is normalised and staged once,
     // and the CTAs' row shares are cut from both matrices together, so that the pipeline ramps up and drains once.
@@ -2487,6 +2759,7 @@ struct Lowerer {
         }
         if (pending_merge.buffer_id >= 0) throw Error(E_INTERNAL, "decode attention merge was left without its consumer");
         if (pending_sum.buffer_id >= 0 && !pending_sum.stored) throw Error(E_INTERNAL, "one-shot all_reduce sum was left without a consumer");
+        fuse_row_chains();
         elide_syncs();
         pair_weight_streams();
         plan_prefetch();

@@ -40,6 +40,7 @@ enum StageKind : int32_t {
     SK_DECODE_ATTN = 15,    // one query row per head against a K/V cache: scores, softmax and output in one pass over the cache
     SK_PACKET = 16,         // flag-carrying packets: local data -> a peer's packet buffer, or local packet buffer -> local data
     SK_PACKET_REDUCE = 17,  // own shard + the shards the peers sent (packets or plain) -> local output and every peer's output
+    SK_ROWCHAIN = 19,       // a run of row-local operators: each row stays in registers from one to the next
     SK_PREFILL_ATTN = 18,   // many query rows per head: S = Q K^T, online softmax and O = P V per 128-row tile, scores stay on chip
 };
 
@@ -112,6 +113,43 @@ struct RowOpArgs {
     int32_t weight_f32;    // 1: `weight` holds fp32 values whatever the rows' type (the llama example keeps its norm weights in fp32)
     int32_t weight_smem;   // staged form: the CTA copies the weight row into shared memory (behind the row buffers) once,
                            // instead of every warp fetching it from L2 a vector at a time for every row
+};
+
+// A run of operators on dense [rows, cols] tensors of one type in which each one works on the result of the one
+// before. Every result is stored as the separate operators would store it; what falls away are the reads of it, the
+// barriers and the stages.
+enum RowChainHead : int32_t {
+    RH_LOAD = 0,   // the row of `src`
+    RH_GATHER = 1, // row idx[row] of `src` (an Embedding), stored to `out`
+    RH_SUM = 2,    // the sum of a matmul's split-K partials (+ `add`, activation), stored to `out`
+};
+enum RowChainKind : int32_t { RC_EWISE = 0, RC_RMSNORM = 1, RC_LAYERNORM = 2, RC_SOFTMAX = 3, RC_CAST = 4 };
+struct RowChainOp {
+    int32_t kind;
+    int32_t op;           // RC_EWISE: EwiseOp; RC_CAST: the result's type
+    int32_t other_mode;   // second operand: 0 none, 1 tensor, 2 one row for all, 3 the value itself
+    int32_t swapped;      // 1: the value is the second operand, `other` the first
+    const void *other;    // RC_RMSNORM: residual added first
+    void *out;
+    void *out2;           // RC_RMSNORM with residual: where the sum goes
+    void *copy;           // optional second place for the result (an equal operator elsewhere in the plan)
+    const void *weight;   // RC_RMSNORM
+    float scalar;         // RC_EWISE: scalar; norms: epsilon; RC_SOFTMAX: scale
+    int32_t weight_f32;
+};
+constexpr int kMaxChainOps = 10;
+struct RowChainArgs {
+    int32_t head, dtype, n_ops, warps;  // warps that share a row (or segment)
+    int32_t rows, cols;                 // cols: of a segment
+    int32_t segs, splits;               // segments per row (1 when an operator needs whole rows); RH_SUM: partials
+    const void *src;                    // RH_LOAD / RH_GATHER
+    const int32_t *idx;
+    int64_t src_ld, num_emb;            // RH_GATHER: table pitch and rows
+    const float *ws;
+    const void *add;                    // RH_SUM: optional tensor added before the activation
+    void *out;                          // RH_GATHER / RH_SUM
+    int32_t act, pad;
+    RowChainOp ops[kMaxChainOps];
 };
 
 // Shared memory the loop kernel offers a matmul stage for operand ring slots when its epilogue needs no staging
@@ -390,11 +428,13 @@ struct alignas(128) Stage {
     int32_t sync_group;              // SK_SYNC: which barrier counter
     int32_t sync_count;              // SK_SYNC: CTAs taking part
     int32_t sync_ord;                // SK_SYNC: 1-based ordinal of this barrier within an iteration
-    int32_t pad0;
+    int32_t work;                    // > 0: only the first `work` processors of the range have a share of this stage; the others
+                                     // do not enter its function (an idle pass through one costs microseconds of register saves)
     union {
         EwiseArgs ew;
         ReduceArgs rd;
         RowOpArgs ro;
+        RowChainArgs rc;
         GemmArgs gm;
         GemvArgs gv;
         DecodeAttnArgs da;

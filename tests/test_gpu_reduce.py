@@ -257,3 +257,100 @@ def test_rmsnorm_with_residual(dt, rows, cols):
     assert np.array_equal(got_x1.view(np.uint16), want_x1.view(np.uint16))
     tol = 2e-3 if dt == "fp16" else 1.6e-2
     assert_close(got_h, O.rmsnorm(want_x1, w, dt, 1e-5), dt, rtol=tol, atol=tol, what=f"rmsnorm + residual {rows}x{cols}")
+
+
+# ---- row chains: operators that follow each other on the same rows run as one stage ----
+def _chain_model(rows, cols, dt):
+    """Embedding, tensor and row operands on either side, all norms, a residual, softmax and a cast."""
+    t = NAME[dt]
+    ids, table = ark.tensor([rows], ark.int32), ark.tensor([50, cols], t)
+    pos, gain, weight = ark.tensor([rows, cols], t), ark.tensor([1, cols], t), ark.tensor([cols], t)
+    e = ark.reshape(ark.embedding(ids, table), [rows, cols])
+    x = ark.sub(pos, e)
+    n = ark.layernorm(x)
+    m = ark.mul(gain, n)
+    g = ark.gelu(m)
+    y, s = ark.rmsnorm(g, weight, residual=x)
+    d = ark.mul(y, y)
+    r = ark.relu(ark.add(d, -0.5))
+    p = ark.softmax(r, scale=0.25)
+    c = ark.cast(p, ark.bf16 if dt == "fp32" else ark.fp32)
+    return dict(ids=ids, table=table, pos=pos, gain=gain, weight=weight), dict(e=e, x=x, n=n, m=m, g=g, y=y, s=s, d=d, r=r, p=p, c=c)
+
+
+@pytest.mark.parametrize("dt", ["fp32", "fp16", "bf16"])
+@pytest.mark.parametrize("rows,cols", [(1, 8), (3, 256), (130, 264), (2400, 1024), (5, 4104), (40, 8192), (2, 16384)])
+def test_row_chain_leaves_every_result(dt, rows, cols):
+    """Each stored result against the float64 operator on the stored operands: one fp32 evaluation and one rounding."""
+    rng = np.random.default_rng(71)
+    ark.init()
+    ins, outs = _chain_model(rows, cols, dt)
+    f = lambda *shape: O.to_storage(rng.normal(0, 1, shape).astype(np.float32), dt)
+    a = dict(ids=rng.integers(-50, 50, rows).astype(np.int32), table=f(50, cols), pos=f(rows, cols), gain=f(1, cols), weight=f(cols))
+    got = dict(zip(outs, execute(list(outs.values()), {ins[k]: v for k, v in a.items()})))
+    w = {k: O.to_f32(v, ("bf16" if dt == "fp32" else "fp32") if k == "c" else dt).astype(np.float64) for k, v in got.items()}
+    i = {k: O.to_f32(v, dt).astype(np.float64) for k, v in a.items() if k != "ids"}
+    assert np.array_equal(w["e"].reshape(rows, cols), i["table"][a["ids"]])  # negative ids count from the end
+    one = 2.0 ** -24
+    half_ulp = {"fp32": one, "fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt]
+    tiny = {"fp32": 2.0 ** -126, "fp16": 2.0 ** -25, "bf16": 2.0 ** -126}[dt]  # subnormals: half of fp16's spacing; may be flushed
+
+    def check(name, want, steps, scale=None, below=0.0):
+        """`steps` fp32 roundings relative to `scale` (default: the result itself), then one to the storage type."""
+        bound = half_ulp * np.abs(want) * 1.01 + steps * one * (np.abs(want) if scale is None else scale) + tiny + below
+        assert (np.abs(w[name] - want) <= bound).all(), name
+
+    check("x", i["pos"] - w["e"].reshape(rows, cols), 0)
+    mean, x = w["x"].mean(1, keepdims=True), w["x"]
+    inv = 1 / np.sqrt(((x - mean) ** 2).mean(1, keepdims=True) + 1e-5)
+    check("n", (x - mean) * inv, cols, (np.abs(x) + np.abs(x).mean(1, keepdims=True)) * inv)
+    check("m", w["n"] * i["gain"], 1)
+    u = 0.7978845608028654 * (w["m"] + 0.044715 * w["m"] ** 3)
+    # fast exponential and reciprocal on 16-bit results; where exp(-2u) overflows, the result 0 stands for less than |m| / 2^128
+    check("g", w["m"] / (1 + np.exp(-2 * u)), 64 * (1 + np.abs(u)), below=np.abs(w["m"]) * 2.0 ** -127)
+    check("s", w["g"] + x, 0)
+    check("y", w["s"] / np.sqrt((w["s"] ** 2).mean(1, keepdims=True) + 1e-5) * i["weight"], cols)
+    check("d", w["y"] ** 2, 1)
+    assert np.array_equal(got["r"], got["r"])
+    check("r", np.maximum(O.to_f32(O.to_storage((w["d"] - 0.5).astype(np.float32), dt), dt), 0), 1, 1 + np.abs(w["d"]))
+    z = w["r"] * 0.25
+    ez = np.exp(z - z.max(1, keepdims=True))
+    check("p", ez / ez.sum(1, keepdims=True), cols + 64 * (1 + z.max() - z.min()))
+    assert np.array_equal(w["c"], w["p"] if dt != "fp32" else O.to_f32(O.to_storage(w["p"].astype(np.float32), "bf16"), "bf16"))
+
+
+@pytest.mark.parametrize("dt", ["fp32", "fp16", "bf16"])
+@pytest.mark.parametrize("rows,cols", [(7, 320), (9000, 256), (600, 4096)])
+def test_elementwise_row_chain_matches_separate_stages(dt, rows, cols, monkeypatch):
+    """Without a reduction the chain may cut rows into segments; the bits are those of the separate stages."""
+    rng = np.random.default_rng(72)
+    f = lambda *shape: O.to_storage(rng.normal(0, 3, shape).astype(np.float32), dt)
+    a, b, row = f(rows, cols), f(rows, cols), f(1, cols)
+    a.flat[:3], b.flat[1:4] = O.to_storage(np.array([np.inf, -np.inf, np.nan], np.float32), dt), O.to_storage(np.array([0, np.inf, 1], np.float32), dt)
+
+    def run():
+        ark.init()
+        ta, tb, tr = (ark.tensor(list(v.shape), NAME[dt]) for v in (a, b, row))
+        x = ark.div(tr, ta)
+        y = ark.silu(ark.add(tb, x))
+        z = ark.mul(y, x)
+        ark.sigmoid(z, output=z)
+        return execute([x, y, z], {ta: a, tb: b, tr: row})
+
+    fused = run()
+    monkeypatch.setenv("ARKB_KEEP_SYNCS", "1")
+    for p, q in zip(fused, run()):
+        assert np.array_equal(O.to_f32(p, dt), O.to_f32(q, dt), equal_nan=True)
+
+
+@pytest.mark.parametrize("rows,cols", [(8192, 512), (4096, 24), (300, 2056)])
+def test_reduce_rows_over_many_segments(rows, cols):
+    rng = np.random.default_rng(73)
+    x = rng.normal(0, 1, (rows, cols)).astype(np.float32)
+    ark.init()
+    t = ark.tensor([rows, cols], ark.fp32)
+    s, m = ark.reduce_sum(t, axis=0), ark.reduce_max(t, axis=0)
+    gs, gm = execute([s, m], {t: x})
+    x64 = x.astype(np.float64)
+    assert (np.abs(gs.reshape(-1) - x64.sum(0)) <= rows * 2.0 ** -24 * np.abs(x64).sum(0)).all()
+    assert np.array_equal(gm.reshape(-1), x.max(0))

@@ -4,14 +4,29 @@
 // The reference builds this from two Matmuls, a scale and a softmax
 // (examples/llama/model.py:336-444), i.e. several tasks with barriers between
 // them; at one query row per head those tasks are nothing but a read of the
-// cache, so this stage does the whole thing around that read:
-//   phase 0  a CTA takes one (sequence, K/V head, chunk of the cache): scores of
-//            the chunk for the G query heads (half a warp per key, fp32), their
-//            maximum and exp-sum, and the chunk's un-normalised output; written
-//            to scratch as fp32 (output, maximum, sum);
-//   phase 1  after a barrier, the chunks of a head are merged with the usual
-//            max/sum rescaling and the result is rounded once.
-// K and V are read exactly once, 16 bytes per lane, rows contiguous.
+// cache, so this stage does the whole thing around that read.
+//
+// What bounds it is HBM. Three things used to keep it a factor of five away (16 sequences of 4096 keys, 64 / 8 heads:
+// 202 us for 268 MB): the multiply-adds of 8 query heads on the CUDA cores, phases of a CTA (scores, softmax, output)
+// that waited for one another with the memory idle, and whole chunks handed to CTAs, so that 160 chunks on 148 CTAs took
+// two rounds. Here:
+//  * The cache is a list of 16-key blocks, (sequence, K/V head) by (sequence, K/V head), cut into runs of equal length,
+//    one per CTA. The pieces of a head (one from each run that holds some of it) are merged afterwards: fp32 output,
+//    maximum and exp-sum per piece.
+//  * Every warp works alone on every 12th block of a run: the scores of 16 keys x 8 heads and the output are 24 small
+//    tensor-core products (mma.sync m16n8k16: with 8 columns of queries there is nothing a larger tile could fill), an
+//    online softmax sits in between, and no warp waits for another one until the piece is complete.
+//  * Probabilities stay at fp32 accuracy: each is the sum of two 16-bit values, its rounding and the remainder, which
+//    take the two row halves of the same product (heads are 8 of the 16 rows). They are scaled by 2^14, which cancels in
+//    the division by their sum, so that fp16 remainders stay clear of the subnormals.
+//  * K and V go through shared memory only as a queue: a lane brings in exactly the 16-byte pieces that it will use as
+//    operand fragments (the head dimension may be permuted alike in K and Q, or in V and the output), a block of K and
+//    one of V ahead.
+// One B200, bf16: 16 sequences of 4096 keys, 64 / 8 heads 202 -> 75 us (3.6 TB/s); 5 sequences of 1337 keys, 32 heads
+// 57 -> 38 us.
+#include <type_traits>
+
+#include "dev_attn.cuh"
 #include "dev_common.cuh"
 #include "dev_funcs.h"
 
@@ -19,25 +34,253 @@ namespace arkb {
 
 namespace {
 
-constexpr int kHeadDim = 128;     // elements per head (16 lanes x 8)
-constexpr int kMaxGroup = 8;      // query heads per K/V head
+constexpr int kHeadDim = 128;
+constexpr int kMaxGroup = 8;                  // query heads per K/V head
+constexpr int kWarps = 12;                    // warps that take part: 96 KiB of queues, with 48 to 96 KiB on their way
+constexpr int kDepth = 2;                     // blocks in a warp's queue: one of K, one of V
+constexpr int kBlockBytes = 16 * kHeadDim * 2;
+constexpr int kRingBytes = kWarps * kDepth * kBlockBytes;
+constexpr int kQBytes = kMaxGroup * kHeadDim * 2;
+constexpr int kRedBytes = kWarps * kMaxGroup * kHeadDim * 4;  // warps' outputs; over the queues, which are empty by then
+static_assert(kRedBytes <= kRingBytes, "the warps' outputs reuse the queues");
+static_assert(kRingBytes + kQBytes + 2 * kWarps * kMaxGroup * 4 <= kDecodeAttnSmemBytes, "shared memory of the stage");
 
+__device__ __forceinline__ void fetch16(uint32_t dst, const void *src, const void *any, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(in ? src : any), "r"(in ? 16 : 0)
+                 : "memory");
+}
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int LEFT>
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(LEFT) : "memory"); }
+__device__ __forceinline__ uint4 lds16(uint32_t a) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(a) : "memory");
+    return v;
+}
 
+template <typename T>
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    if constexpr (std::is_same_v<T, __nv_bfloat16>)
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+    else
+        asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+            : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+// 8 x 8 matrix of 16-bit values, a row per four lanes, transposed across the warp
+__device__ __forceinline__ uint32_t transpose8x8(uint32_t v) {
+    uint32_t r;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(r) : "r"(v));
+    return r;
+}
+template <typename T>
+__device__ __forceinline__ uint32_t pack2(T a, T b) {
+    uint32_t r;
+    T *e = reinterpret_cast<T *>(&r);
+    e[0] = a;
+    e[1] = b;
+    return r;
+}
+constexpr float kLowest = -3.402823466e+38f;
+constexpr float kLog2e = 1.4426950408889634f;
+
+template <typename T>
+__device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *smem) {
+    T *qs = reinterpret_cast<T *>(smem + kRingBytes);                      // [8][128], rows of absent heads zero
+    float *wm = reinterpret_cast<float *>(smem + kRingBytes + kQBytes);    // [warp][8]: maximum (log2 units), then exp-sum
+    float *wl = wm + kWarps * kMaxGroup;
+    float *red = reinterpret_cast<float *>(smem);                          // [warp][G][128]
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int g = lane >> 2, t = lane & 3;                                 // row group and place in it of the fragments
+    const int G = a.Hq / a.Hkv, nb = a.pieces.blocks;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(smem) + warp * (kDepth * kBlockBytes) + lane * 16;
+    const float to_log2 = a.scale * kLog2e;
+    const int run0 = a.pieces.begin(p), run1 = p + 1 < a.pieces.runs ? a.pieces.begin(p + 1) : a.B * a.Hkv * nb;
+    for (int blk = run0; blk < run1;) {
+        const int head = blk / nb, kb0 = blk - head * nb, kb1 = min(nb, kb0 + run1 - blk);  // blocks [kb0, kb1) of this head
+        blk += kb1 - kb0;
+        const int kvh = head % a.Hkv, b = head / a.Hkv;
+        const T *kbase = reinterpret_cast<const T *>(a.k) + (int64_t)b * a.k_stride_b + (int64_t)kvh * a.k_stride_h;
+        const T *vbase = reinterpret_cast<const T *>(a.v) + (int64_t)b * a.v_stride_b + (int64_t)kvh * a.v_stride_h;
+        const int n_mine = kb1 - kb0 > warp ? (kb1 - kb0 - warp + kWarps - 1) / kWarps : 0;
+        // K of a block: rows g and g + 8, 16 bytes at 32 i + 8 t. V: rows 2 t, 2 t + 1, 2 t + 8, 2 t + 9, 16 bytes at 64 h + 8 g.
+        auto fetch_k = [&](int i) {
+            if (i < n_mine) {
+                const int key = (kb0 + warp + i * kWarps) * 16 + g;
+#pragma unroll
+                for (int c = 0; c < 8; ++c)
+                    fetch16(ring + c * 512, kbase + (int64_t)(key + (c & 1) * 8) * a.k_ld + (c >> 1) * 32 + t * 8, kbase,
+                            key + (c & 1) * 8 < a.T);
+            }
+            fetch_commit();
+        };
+        auto fetch_v = [&](int i) {
+            if (i < n_mine) {
+                const int key = (kb0 + warp + i * kWarps) * 16 + 2 * t;
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    const int r = key + (c & 1) + (c >> 1 & 1) * 8;
+                    fetch16(ring + kBlockBytes + c * 512, vbase + (int64_t)r * a.v_ld + (c >> 2) * 64 + g * 8, vbase, r < a.T);
+                }
+            }
+            fetch_commit();
+        };
+        named_barrier(1, kWarps * 32);  // the queues' memory is no longer read as the outputs of the piece before
+        fetch_k(0);
+        fetch_v(0);
+        const T *qb = reinterpret_cast<const T *>(a.q) + (int64_t)b * a.q_stride_b + (int64_t)kvh * G * a.q_stride_h;
+        if (tid < kMaxGroup * kHeadDim / 8) {
+            const int h = tid >> 4, v = tid & 15;
+            uint4 q4 = make_uint4(0, 0, 0, 0);
+            if (h < G) {
+                q4 = *reinterpret_cast<const uint4 *>(qb + (int64_t)h * a.q_stride_h + v * 8);
+                if (a.rope) {
+                    // rotary embedding of the new token's query (complex multiply of adjacent pairs with the position's
+                    // (cos, sin) pairs), rounded like the separate operator would have stored it
+                    float f[8], c[8];
+                    unpack8<T>(q4, f);
+                    unpack8<T>(*reinterpret_cast<const uint4 *>(reinterpret_cast<const T *>(a.rope) + v * 8), c);
+                    T *e = reinterpret_cast<T *>(&q4);
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        e[i] = from_f32<T>(f[i] * c[i] - f[i + 1] * c[i + 1]);
+                        e[i + 1] = from_f32<T>(f[i] * c[i + 1] + f[i + 1] * c[i]);
+                    }
+                }
+            }
+            *reinterpret_cast<uint4 *>(qs + h * kHeadDim + v * 8) = q4;
+        }
+        named_barrier(1, kWarps * 32);
+        uint4 qf[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) qf[i] = *reinterpret_cast<const uint4 *>(qs + g * kHeadDim + i * 32 + t * 8);
+        float o[16][4] = {};                       // [n-tile 8 h + j]: rows g (rounded probabilities) and g + 8 (remainders)
+        float m0 = kLowest, m1 = kLowest, l0 = 0.0f, l1 = 0.0f;  // heads 2 t and 2 t + 1
+        for (int i = 0; i < n_mine; ++i) {
+            fetch_wait<1>();  // K of block i; V of block i is on its way
+            float c[4] = {}, d[4] = {};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint4 x = lds16(ring + k * 1024), y = lds16(ring + k * 1024 + 512);
+                mma16816<T>(c, x.x, y.x, x.y, y.y, qf[k].x, qf[k].y);
+                mma16816<T>(d, x.z, y.z, x.w, y.w, qf[k].z, qf[k].w);
+            }
+            fetch_k(i + 1);
+            const int key = (kb0 + warp + i * kWarps) * 16 + g;
+            const bool in0 = key < a.T, in1 = key + 8 < a.T;
+            const float s0 = in0 ? (c[0] + d[0]) * to_log2 : -INFINITY, s1 = in0 ? (c[1] + d[1]) * to_log2 : -INFINITY;
+            const float s2 = in1 ? (c[2] + d[2]) * to_log2 : -INFINITY, s3 = in1 ? (c[3] + d[3]) * to_log2 : -INFINITY;
+            float x0 = fmaxf(s0, s2), x1 = fmaxf(s1, s3);
+#pragma unroll
+            for (int w = 4; w < 32; w *= 2) {
+                x0 = fmaxf(x0, __shfl_xor_sync(0xffffffffu, x0, w));
+                x1 = fmaxf(x1, __shfl_xor_sync(0xffffffffu, x1, w));
+            }
+            x0 = fmaxf(x0, m0);
+            x1 = fmaxf(x1, m1);
+            if (__any_sync(0xffffffffu, x0 > m0 || x1 > m1)) {
+                const float f0 = exp2_fast(m0 - x0), f1 = exp2_fast(m1 - x1);
+                l0 *= f0;
+                l1 *= f1;
+                m0 = x0;
+                m1 = x1;
+                // the output's rows are heads g: their factors are with the lanes whose t is g / 2
+                const float e0 = __shfl_sync(0xffffffffu, f0, g >> 1), e1 = __shfl_sync(0xffffffffu, f1, g >> 1);
+                const float f = g & 1 ? e1 : e0;
+#pragma unroll
+                for (int n = 0; n < 16; ++n)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[n][e] *= f;
+            }
+            const float p0 = exp2_fast(s0 - m0 + 14.0f), p1 = exp2_fast(s1 - m1 + 14.0f);
+            const float p2 = exp2_fast(s2 - m0 + 14.0f), p3 = exp2_fast(s3 - m1 + 14.0f);
+            l0 += p0 + p2;
+            l1 += p1 + p3;
+            const T h0 = from_f32<T>(p0), h1 = from_f32<T>(p1), h2 = from_f32<T>(p2), h3 = from_f32<T>(p3);
+            const uint32_t a0 = transpose8x8(pack2<T>(h0, h1)), a2 = transpose8x8(pack2<T>(h2, h3));
+            const uint32_t a1 = transpose8x8(pack2<T>(from_f32<T>(p0 - to_f32(h0)), from_f32<T>(p1 - to_f32(h1))));
+            const uint32_t a3 = transpose8x8(pack2<T>(from_f32<T>(p2 - to_f32(h2)), from_f32<T>(p3 - to_f32(h3))));
+            fetch_wait<1>();
+            const uint32_t vs = ring + kBlockBytes;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const uint4 v0 = lds16(vs + h * 2048), v1 = lds16(vs + h * 2048 + 512), v2 = lds16(vs + h * 2048 + 1024), v3 = lds16(vs + h * 2048 + 1536);
+                const uint32_t r0[4] = {v0.x, v0.y, v0.z, v0.w}, r1[4] = {v1.x, v1.y, v1.z, v1.w};
+                const uint32_t r2[4] = {v2.x, v2.y, v2.z, v2.w}, r3[4] = {v3.x, v3.y, v3.z, v3.w};
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    mma16816<T>(o[h * 8 + 2 * r], a0, a1, a2, a3, __byte_perm(r0[r], r1[r], 0x5410), __byte_perm(r2[r], r3[r], 0x5410));
+                    mma16816<T>(o[h * 8 + 2 * r + 1], a0, a1, a2, a3, __byte_perm(r0[r], r1[r], 0x7632), __byte_perm(r2[r], r3[r], 0x7632));
+                }
+            }
+            fetch_v(i + 1);
+        }
+        fetch_wait<0>();
+        // the warps' pieces become one: common maximum, rescaled sums and outputs
+#pragma unroll
+        for (int w = 4; w < 32; w *= 2) {
+            l0 += __shfl_xor_sync(0xffffffffu, l0, w);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, w);
+        }
+        if (g == 0) {
+            wm[warp * kMaxGroup + 2 * t] = m0;
+            wm[warp * kMaxGroup + 2 * t + 1] = m1;
+            wl[warp * kMaxGroup + 2 * t] = l0;
+            wl[warp * kMaxGroup + 2 * t + 1] = l1;
+        }
+        named_barrier(1, kWarps * 32);
+        if (g < G) {
+            float m = kLowest;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) m = fmaxf(m, wm[w * kMaxGroup + g]);
+            const float f = exp2_fast(wm[warp * kMaxGroup + g] - m);
+            float *dst = red + (warp * G + g) * kHeadDim + 16 * t;
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {  // columns 2 t and 2 t + 1 of n-tile j are elements 16 t + j and 16 t + 8 + j of the half
+                    dst[h * 64 + j] = (o[h * 8 + j][0] + o[h * 8 + j][2]) * f;
+                    dst[h * 64 + 8 + j] = (o[h * 8 + j][1] + o[h * 8 + j][3]) * f;
+                }
+        }
+        named_barrier(1, kWarps * 32);
+        float *out = a.ws + a.pieces.record(p, head) * G * (kHeadDim + 4);
+        for (int i = tid; i < G * kHeadDim; i += kWarps * 32) {
+            float s = 0.0f;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) s += red[w * G * kHeadDim + i];
+            out[i] = s;
+        }
+        if (tid < G) {
+            float m = kLowest, l = 0.0f;
+            for (int w = 0; w < kWarps; ++w) m = fmaxf(m, wm[w * kMaxGroup + tid]);
+            for (int w = 0; w < kWarps; ++w) l += wl[w * kMaxGroup + tid] * exp2_fast(wm[w * kMaxGroup + tid] - m);
+            out[G * kHeadDim + 2 * tid] = m;
+            out[G * kHeadDim + 2 * tid + 1] = l;
+        }
+    }
+}
+
+// One or two sequences: a CTA takes one (sequence, K/V head, chunk of the cache): scores of the chunk for the G query heads
+// (half a warp per key, fp32), their maximum and exp-sum, and the chunk's un-normalised output. As fast as the block form
+// above where each processor sees few keys (one sequence of 2048 keys, 32 heads: 16.5 us both), and it takes 11 KiB of
+// shared memory instead of 102: the matmuls of such a plan stream their weights through L1, and each of them ran 1 to 4 us
+// longer beside the larger one (4 layers: 537 us against 577).
 template <typename T, int G>
 __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, char *smem) {
     constexpr int D = kHeadDim;
     float *qs = reinterpret_cast<float *>(smem);                 // [G][D], already scaled
-    float *ml = qs + G * D;                                      // [G][2]: maximum, exp-sum
+    float *ml = qs + G * D;                                      // [G][2]: maximum (log2 units), exp-sum
     float *sc = ml + 2 * kMaxGroup;                              // [G][chunk_len]
     float *red = sc + (size_t)G * a.chunk_len;                   // [16][G][D]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int hw = tid >> 4, l16 = tid & 15;                     // half-warp index 0..31, lane within it
-    const int items = a.B * a.Hkv * a.chunks;
+    const int chunks = a.pieces.per_span, items = a.B * a.Hkv * chunks;
     const T *qb = reinterpret_cast<const T *>(a.q);
     const T *kb = reinterpret_cast<const T *>(a.k);
     const T *vb = reinterpret_cast<const T *>(a.v);
     for (int item = p; item < items; item += P) {
-        const int c = item % a.chunks, bh = item / a.chunks;
+        const int c = item % chunks, bh = item / chunks;
         const int kvh = bh % a.Hkv, b = bh / a.Hkv;
         const int t0 = c * a.chunk_len, len = min(a.chunk_len, a.T - t0);
         __syncthreads();  // the previous item's shared memory is no longer read
@@ -110,7 +353,7 @@ __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, 
             }
             l = warp_sum(l);
             if (lane == 0) {
-                ml[warp * 2] = m;
+                ml[warp * 2] = m * kLog2e;
                 ml[warp * 2 + 1] = l;
             }
         }
@@ -159,7 +402,7 @@ __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, 
             }
         }
         __syncthreads();
-        float *w = a.ws + (size_t)item * G * (D + 2);
+        float *w = a.ws + (size_t)item * G * (D + 4);
         const int nwarps = blockDim.x >> 5;
         for (int i = tid; i < G * D; i += blockDim.x) {
             float s = 0.0f;
@@ -170,40 +413,31 @@ __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, 
     }
 }
 
-// Merges the chunks of every (sequence, query head): thread per output element.
+// Merges the pieces of every (sequence, query head): thread per output element.
 template <typename T>
 __device__ void attn_merge(const DecodeAttnArgs &a, int p, int P) {
     constexpr int D = kHeadDim;
-    const int G = a.Hq / a.Hkv;
-    const int64_t total = (int64_t)a.B * a.Hq * D;
+    const int G = a.Hq / a.Hkv, total = a.B * a.Hq * D;
     T *out = reinterpret_cast<T *>(a.out);
-    for (int64_t i = (int64_t)p * blockDim.x + threadIdx.x; i < total; i += (int64_t)P * blockDim.x) {
-        const int d = (int)(i % D);
-        const int h = (int)((i / D) % a.Hq), b = (int)(i / ((int64_t)D * a.Hq));
-        const int kvh = h / G, g = h % G;
-        const float *w = a.ws + ((size_t)(b * a.Hkv + kvh) * a.chunks) * G * (D + 2);
-        const size_t stride = (size_t)G * (D + 2);
-        float m = -3.402823466e+38f;
-        for (int c = 0; c < a.chunks; ++c) m = fmaxf(m, w[c * stride + G * D + 2 * g]);
-        float l = 0.0f, o = 0.0f;
-        for (int c = 0; c < a.chunks; ++c) {
-            const float f = __expf(w[c * stride + G * D + 2 * g] - m);
-            l += w[c * stride + G * D + 2 * g + 1] * f;
-            o += w[c * stride + g * D + d] * f;
-        }
-        out[(int64_t)b * a.o_stride_b + (int64_t)h * a.o_stride_h + d] = from_f32<T>(o / l);
+    for (int i = p * (int)blockDim.x + threadIdx.x; i < total; i += P * (int)blockDim.x) {
+        const int d = i % D, h = i / D % a.Hq, b = i / (D * a.Hq);
+        float l, o[1];
+        merge_pieces<1>(a.pieces, a.ws, b * a.Hkv + h / G, G, h % G, d, l, o);
+        out[(int64_t)b * a.o_stride_b + (int64_t)h * a.o_stride_h + d] = from_f32<T>(o[0] / l);
     }
 }
 
 template <typename T>
-__device__ void attn_typed(const DecodeAttnArgs &a, int p, int P, char *smem) {
-    if (a.phase == 1) return attn_merge<T>(a, p, P);
-    switch (a.Hq / a.Hkv) {
-        case 1: return attn_chunks<T, 1>(a, p, P, smem);
-        case 2: return attn_chunks<T, 2>(a, p, P, smem);
-        case 4: return attn_chunks<T, 4>(a, p, P, smem);
-        default: return attn_chunks<T, 8>(a, p, P, smem);
-    }
+__device__ __forceinline__ void attn_typed(const DecodeAttnArgs &a, int p, int P, char *smem) {
+    if (a.phase == 1) attn_merge<T>(a, p, P);
+    else if (a.chunk_len > 0) {
+        switch (a.Hq / a.Hkv) {
+            case 1: return attn_chunks<T, 1>(a, p, P, smem);
+            case 2: return attn_chunks<T, 2>(a, p, P, smem);
+            case 4: return attn_chunks<T, 4>(a, p, P, smem);
+            default: return attn_chunks<T, 8>(a, p, P, smem);
+        }
+    } else if (p < a.pieces.runs && threadIdx.x < kWarps * 32) attn_pieces<T>(a, p, smem);
 }
 
 }  // namespace

@@ -19,6 +19,7 @@
 // ws[range][m][n] and the split-K sum stage that follows adds them in range
 // order, applies the activation and rounds (deterministic).
 #include "dev_comm.cuh"
+#include "dev_attn.cuh"
 #include "dev_common.cuh"
 #include "dev_funcs.h"
 
@@ -98,7 +99,7 @@ __device__ __forceinline__ void load_x8(const GemvArgs &a, const PushTo &c, int 
         // the attention's chunks of head k / 128 of sequence m, merged with the usual max / sum rescaling and rounded
         // like the merge stage would have stored them
         const int G = a.mg_group, h = k >> 7, d = k & 127, kvh = h / G, g = h % G;
-        const size_t stride = (size_t)G * 130;
+        const size_t stride = (size_t)G * 132;
         const float *w = reinterpret_cast<const float *>(a.pro_a) + ((size_t)(m * a.mg_kv_heads + kvh) * a.mg_chunks) * stride;
         float mx = -3.402823466e+38f;
         for (int c = 0; c < a.mg_chunks; ++c) mx = fmaxf(mx, w[c * stride + G * 128 + 2 * g]);
@@ -106,9 +107,9 @@ __device__ __forceinline__ void load_x8(const GemvArgs &a, const PushTo &c, int 
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = 0.0f;
         for (int c = 0; c < a.mg_chunks; ++c) {
-            const float e = __expf(w[c * stride + G * 128 + 2 * g] - mx);
+            const float e = exp2_fast(w[c * stride + G * 128 + 2 * g] - mx);  // maxima are in log2 units
             l += w[c * stride + G * 128 + 2 * g + 1] * e;
-            const float2 *o = reinterpret_cast<const float2 *>(w + c * stride + g * 128 + d);  // records are 8-byte aligned
+            const float2 *o = reinterpret_cast<const float2 *>(w + c * stride + g * 128 + d);
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
                 const float2 v = o[i];

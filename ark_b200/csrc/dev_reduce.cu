@@ -149,7 +149,7 @@ __device__ void reduce_other_axis(const ReduceArgs &a, int p, int P, float *red)
     // With fewer output vectors than threads, S threads of a CTA share one output vector: each walks 1/S of the
     // reduced axis and the partial results are added through shared memory (a fixed tree: deterministic). Up to 128
     // segments, so that 4 neighbouring vectors (64 bytes of a row) are the least a CTA takes: 8192 rows of 4096 bf16 are
-    // 512 vectors, which 16 segments left to 16 CTAs (90 us), 128 spread over 128 (@@RED@@).
+    // 512 vectors, which 16 segments left to 16 CTAs (90 us), 128 spread over 128 (25 us).
     int S = 1;
     while (S < 128 && units * S * 2 <= (int64_t)P * kThreads && len / (S * 2) >= 16) S *= 2;
     const int UPB = kThreads / S;  // output vectors per CTA pass

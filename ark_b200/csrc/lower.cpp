@@ -534,7 +534,7 @@ struct Lowerer {
     bool gemv_pushed = false;  // set by lower_matmul when the push of a one-shot all_reduce was folded in
     // Operators folded across processor groups in the decode chain:
     const OpDesc *rope_for_attention = nullptr;  // a Rope whose only reader is the DecodeAttention of the next group
-    struct PendingMerge {                        // a DecodeAttention whose chunks the weight-streaming matmul of the next group merges
+    struct PendingMerge {                        // a DecodeAttention whose pieces the weight-streaming matmul of the next group merges
         int64_t buffer_id = -1;
         const float *ws = nullptr;
         size_t ws_bytes = 0;
@@ -1019,7 +1019,7 @@ struct Lowerer {
                 const int64_t per_block = 16 * 1024 + b_rows_k * 128;
                 int G = 1;
                 if (K % 64 == 0) {
-                    if (kSwappedRingBytes / (2 * per_block) >= 4) G = 2;
+                    if (g.tile_n <= 16 || kSwappedRingBytes / (2 * per_block) >= 4) G = 2;
                 }
                 if (const char *e = getenv("ARKB_KGROUP")) G = std::max(1, std::min(G, atoi(e)));
                 g.kgroup = G;
@@ -1216,7 +1216,7 @@ struct Lowerer {
         }
         // ring: 16 KiB A block + this CTA's B block per stage, as many stages as fit in 192 KiB (at most 12)
         g.stage_b_bytes = (int32_t)(g.b_mn_major ? ((b_rows + 63) / 64) * 64 * 128 : b_rows * 128);
-        if (swapped && g.kgroup > 1) g.stages = (int32_t)std::min<int64_t>(12, kSwappedRingBytes / (g.kgroup * (16 * 1024 + g.stage_b_bytes)));
+        if (swapped && g.kgroup > 1) g.stages = (int32_t)std::min<int64_t>(12, (g.tile_n <= 16 ? kFewRowsRingBytes : kSwappedRingBytes) / (g.kgroup * (16 * 1024 + g.stage_b_bytes)));
         else g.stages = (int32_t)std::min<int64_t>(12, (192 * 1024) / ((g.tall ? 32 : 16) * 1024 + g.stage_b_bytes));
         // output through TMA stores of 32x32 blocks: needs 16-byte aligned rows and whole 32-column blocks per tile
         g.c_tma = (!swapped && g.c_vec && g.tile_n % 32 == 0 && (cst[3] * es) % 16 == 0 && (cst[2] * cst[3] * es) % 16 == 0 && !g.bias) ? 1 : 0;
@@ -1335,23 +1335,53 @@ struct Lowerer {
         a.B = (int32_t)B; a.Hq = (int32_t)Hq; a.Hkv = (int32_t)Hkv; a.T = (int32_t)T;
         a.dtype = q.dtype;
         a.scale = op.has_arg("Scale") ? (float)op.arg_float("Scale") : 1.0f;
-        // chunks of the cache: at most two work items per CTA (one more would cost a third round), at least 128 and at
-        // most 2048 keys each; among the candidates the one with the least makespan (rounds x keys per item)
-        const int64_t P = proc.count();
-        const int64_t max_chunks = std::max<int64_t>(1, std::min<int64_t>(2 * P / (B * Hkv), (T + 127) / 128));
-        int64_t chunks = 1, chunk_len = 0;
-        {
-            int64_t best = -1;
+        // 16-key blocks, cut evenly over all processors (a run may then hold the end of one head and the start of the next)
+        // or head by head into as many runs as processors allow. A piece costs about as much as 40 blocks besides its
+        // blocks (start of the stream, sum over the warps: 8 us measured), so 32 heads of 2048 keys are better off with four runs
+        // each on 128 processors, 160 heads of 1337 keys with the even cut.
+        const int64_t P = proc.count(), nb = (T + 15) / 16, heads = B * Hkv, total = heads * nb;
+        if (total > INT32_MAX) throw Error(E_UNSUPPORTED, "DecodeAttention: the cache is too large");
+        AttnPieces &pc = a.pieces;
+        auto cut = [&](int64_t span, int64_t runs_per_span) {
+            pc.blocks = (int32_t)nb;
+            pc.span = (int32_t)span;
+            pc.per_span = (int32_t)runs_per_span;
+            pc.runs = (int32_t)(total / span * runs_per_span);
+            pc.rlen = (int32_t)(span / runs_per_span);
+            pc.rem = (int32_t)(span % runs_per_span);
+            pc.per_run = 1;
+            int64_t most = 0;
+            for (int r = 0; r < pc.runs; ++r) {
+                const int64_t b = pc.begin(r), e = r + 1 < pc.runs ? pc.begin(r + 1) : total, pieces = (e - 1) / nb - b / nb + 1;
+                pc.per_run = std::max<int32_t>(pc.per_run, (int32_t)pieces);
+                most = std::max(most, e - b + 40 * pieces);
+            }
+            return most;
+        };
+        if (B <= kGemvMaxM) {
+            // at most two work items per CTA (one more would cost a third round), at least 128 and at most 2048 keys each;
+            // among the candidates the one with the least makespan (rounds x keys per item)
+            const int64_t max_chunks = std::max<int64_t>(1, std::min<int64_t>(2 * P / heads, (T + 127) / 128));
+            int64_t best = -1, chunks = 1;
             for (int64_t c = 1; c <= max_chunks; ++c) {
                 const int64_t len = std::min<int64_t>(2048, ((T + c - 1) / c + 31) / 32 * 32);
                 const int64_t n = (T + len - 1) / len;
-                const int64_t rounds = (B * Hkv * n + P - 1) / P;
-                const int64_t cost = rounds * (len + 64);  // 64 keys' worth of fixed cost per item
-                if (best < 0 || cost < best) { best = cost; chunks = n; chunk_len = len; }
+                const int64_t cost = (heads * n + P - 1) / P * (len + 64);  // 64 keys' worth of fixed cost per item
+                if (best < 0 || cost < best) { best = cost; chunks = n; a.chunk_len = (int32_t)len; }
             }
+            pc.per_span = (int32_t)chunks;
+            pc.rlen = a.chunk_len / 16;
+            pc.blocks = pc.span = pc.per_span * pc.rlen;
+            pc.rem = 0;
+            pc.per_run = 1;
+            pc.runs = (int32_t)(heads * chunks);
+        } else {
+            const int64_t even = std::min<int64_t>(P, (total + 3) / 4);  // at least 4 blocks, more pieces cost more merging
+            const int64_t per_head = std::min(nb, P / heads);
+            const int64_t cost = cut(total, even);
+            if (per_head >= 1 && cut(nb, per_head) > cost) cut(total, even);
         }
-        a.chunks = (int32_t)chunks; a.chunk_len = (int32_t)chunk_len;
-        const size_t bytes = (size_t)B * Hkv * chunks * G * (128 + 2) * sizeof(float);
+        const size_t bytes = (size_t)pc.runs * pc.per_run * G * (128 + 4) * sizeof(float);
         a.ws = env.workspace ? reinterpret_cast<float *>(env.workspace + prog.workspace_bytes) : nullptr;
         prog.workspace_bytes += (bytes + 255) / 256 * 256;
         a.phase = 0;
@@ -1359,12 +1389,12 @@ struct Lowerer {
         if (rope) { rd(rope->reads[0]); rd(rope->reads[1]); } else rd(q);
         rd_streamed(k); rd_streamed(v);
         wr_raw(a.ws, bytes);
-        s.work = (int32_t)std::min<int64_t>(P, B * Hkv * chunks);
+        s.work = (int32_t)std::min<int64_t>(P, pc.runs);
         push(s, "DecodeAttention " + op.name + " B=" + std::to_string(B) + " heads=" + std::to_string(Hq) + "/" + std::to_string(Hkv) +
-                    " keys=" + std::to_string(T) + " chunks=" + std::to_string(chunks) + " x " + std::to_string(chunk_len) + (rope ? " <-rope" : ""));
+                    " keys=" + std::to_string(T) + (a.chunk_len ? " chunks=" + std::to_string(pc.per_span) + " x " + std::to_string(a.chunk_len) : " blocks=" + std::to_string(total) + " runs=" + std::to_string(pc.runs)) + (rope ? " <-rope" : ""));
         // When the only reader of the result is the weight-streaming matmul of the next processor group (one or two
-        // sequences), that stage merges the chunks while it stages its activations: no merge stage, one barrier less.
-        if (fold_decode_chain() && env.workspace) {
+        // sequences), that stage merges the pieces while it stages its activations: no merge stage, one barrier less.
+        if (fold_decode_chain() && env.workspace && a.chunk_len) {
             const TaskGroup *ntg = nullptr;
             const OpDesc *nx = first_op_of(cur_pg + 1, &ntg);
             if (nx && nx->type == "Matmul" && !nx->reads.empty() && nx->reads[0].buffer_id == o.buffer_id && nx->reads[0].dense() &&
@@ -1372,7 +1402,7 @@ struct Lowerer {
                 other_readers(o.buffer_id, nx) == 0) {
                 pending_merge.buffer_id = o.buffer_id;
                 pending_merge.ws = a.ws; pending_merge.ws_bytes = bytes;
-                pending_merge.chunks = (int)chunks; pending_merge.group = (int)G; pending_merge.kv_heads = (int)Hkv;
+                pending_merge.chunks = pc.per_span; pending_merge.group = (int)G; pending_merge.kv_heads = (int)Hkv;
                 pending_merge.B = B; pending_merge.Hq = Hq;
                 pending_merge_pg = cur_pg;
                 return;
@@ -2528,7 +2558,7 @@ struct Lowerer {
                     erase(j, j + 1);
                 }
             s.rc = best.a;
-            s.work = (int32_t)std::min<int64_t>(prog.grid, ((int64_t)best.a.rows * best.a.segs * best.a.warps + kThreads / 32 - 1) / (kThreads / 32));
+            s.work = (int32_t)std::min<int64_t>(prog.grid, (int64_t)best.a.rows * best.a.segs);
             prog.stages[i] = s;
             prog.access[i] = x;
             prog.notes[i] = note;
@@ -2768,7 +2798,9 @@ struct Lowerer {
         for (auto &s : prog.stages) {
             size_t need = 0;
             switch (s.kind) {
-                case SK_GEMM: need = kFullSmemBytes; break;
+                case SK_GEMM:  // ring alone where the epilogue has no staging area
+                    need = s.gm.out_transposed && s.gm.kgroup > 1 ? (size_t)s.gm.stages * s.gm.kgroup * (16 * 1024 + s.gm.stage_b_bytes) : kFullSmemBytes;
+                    break;
                 case SK_PREFILL_ATTN: need = kFullSmemBytes; break;
                 case SK_GEMM_SIMT: {  // two buffers of k-blocks of both operands for each group of threads, every k padded by 4 floats
                     const size_t tk = s.gs.wm == 1 ? 8 : 16;
@@ -2790,7 +2822,7 @@ struct Lowerer {
                     break;
                 case SK_DECODE_ATTN: {
                     const size_t G = (size_t)(s.da.Hq / std::max(1, s.da.Hkv));
-                    need = (G * 128 + 16 + G * (size_t)s.da.chunk_len + 16 * G * 128) * sizeof(float) + 1024;
+                    if (s.da.phase == 0) need = s.da.chunk_len ? (G * 128 + 16 + G * (size_t)s.da.chunk_len + 16 * G * 128) * sizeof(float) + 1024 : kDecodeAttnSmemBytes;
                     break;
                 }
                 default: break;

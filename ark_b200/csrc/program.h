@@ -155,6 +155,11 @@ struct RowChainArgs {
 // Shared memory the loop kernel offers a matmul stage for operand ring slots when its epilogue needs no staging
 // area (the swapped and split-K forms); stages with a TMA-store epilogue use the first 192 KiB only.
 constexpr int kSwappedRingBytes = 208 * 1024;
+// With at most 16 rows of activations three slots of two k-blocks keep 72 KiB per SM on their way, more than the 53 KiB
+// that HBM's bandwidth and latency ask for, and a plan of such stages leaves half of the SM's memory to L1, where the
+// stage functions' register save areas then stay (five sequences, 7B-shaped, with
+// the attention's queues cut alike: two layers 536 -> 490 us).
+constexpr int kFewRowsRingBytes = 108 * 1024;
 
 struct GemmArgs {
     CUtensorMap tmA;  // dims {inner, rows, C, N}; box {64, 128 or 64, 1, 1}, 128-byte swizzle
@@ -218,6 +223,29 @@ struct SplitKReduceArgs {
     int32_t splits, dtype, act, pad;
 };
 
+// How a decode attention cuts the K/V cache: 16-key blocks, `blocks` per (sequence, K/V head). Every `span` blocks (all of
+// them, or one head's) are cut into `per_span` runs of rlen + 1 (the first `rem`) and rlen blocks; there are `runs` in
+// all, one per processor. The part of a head in a run is a piece; its record (per query head of the group: 128 outputs; then
+// maximum, in log2 units, and exp-sum for each) is number run * per_run + (head - first head of the run).
+struct AttnPieces {
+    int32_t blocks, runs, span, per_span, rlen, rem, per_run;
+#ifdef __CUDACC__
+#define ARKB_HD __host__ __device__
+#else
+#define ARKB_HD
+#endif
+    ARKB_HD int begin(int run) const {
+        const int s = run / per_span, r = run - s * per_span;
+        return s * span + r * rlen + (r < rem ? r : rem);
+    }
+    ARKB_HD int run_of(int block) const {
+        const int s = block / span, b = block - s * span, longer = rem * (rlen + 1);
+        return s * per_span + (b < longer ? b / (rlen + 1) : rem + (b - longer) / rlen);
+    }
+    ARKB_HD int64_t record(int run, int head) const { return (int64_t)run * per_run + (head - begin(run) / blocks); }
+};
+constexpr int kDecodeAttnSmemBytes = 102 * 1024;
+
 struct GemvArgs {
     // y[M, N] = x[M, K] . W with M <= kGemvMaxM on the CUDA cores; W is [N, K] (w_is_nk) or [K, N]
     void *out;        // y, row pitch ldo (written when splits == 1)
@@ -248,9 +276,9 @@ struct GemvArgs {
     int32_t push_ord, push_per_iter;
     uint64_t push_stage_bytes;
     int32_t light;           // [N, K]: the walker with half the loads in flight and a third of the registers (small matrices)
-    // GP_ATTN_MERGE: x is the output of a decode attention whose chunks have not been merged yet: x[b, h * 128 + d] is
-    // put together from the chunk records (pro_a = the attention's scratch: per (b, kv head, chunk) G x (128 outputs +
-    // maximum + sum), fp32) while the activations are staged; M = sequences
+    // GP_ATTN_MERGE: x is the output of a decode attention whose pieces have not been merged yet: x[b, h * 128 + d] is
+    // put together from the chunks' records (pro_a = the attention's scratch: per (b, kv head, chunk) G x 128 outputs, then
+    // maximum and sum for each, fp32, padded to G x 132) while the activations are staged; M = sequences
     int32_t mg_chunks, mg_group, mg_kv_heads;
     // A second matrix of the same shape over the same activations ([N, K] layout, one k-range): rows N .. 2N-1 of the
     // stage's row space are rows of w_b, their results go to out_b with activation act_b (W1 and W3 of a SwiGLU block:
@@ -262,15 +290,16 @@ struct GemvArgs {
 enum GemvPrologue : int32_t { GP_NONE = 0, GP_RMSNORM = 1, GP_MUL = 2, GP_ATTN_MERGE = 3 };
 constexpr int kGemvMaxM = 2;
 
-// softmax(scale * q . K^T) . V for one query row per head (decode); phase 0: per cache chunk, phase 1: merge the chunks
+// softmax(scale * q . K^T) . V for one query row per head (decode); phase 0: the pieces, phase 1: merge them
 struct DecodeAttnArgs {
     void *out;                 // [B, Hq, 1, 128]
     const void *q, *k, *v;     // q [B, Hq, 1, 128]; k, v [B, Hkv, T, 128]
-    float *ws;                 // per (b, kv head, chunk): G x (128 outputs + maximum + sum), fp32
+    float *ws;                 // the pieces' records, fp32
     int64_t q_stride_b, q_stride_h, o_stride_b, o_stride_h;          // elements
     int64_t k_stride_b, k_stride_h, k_ld, v_stride_b, v_stride_h, v_ld;
     int32_t B, Hq, Hkv, T;
-    int32_t chunks, chunk_len;  // the cache is cut into `chunks` pieces of chunk_len keys (a multiple of 32)
+    AttnPieces pieces;
+    int32_t chunk_len;         // > 0: the form for one or two sequences, pieces of chunk_len keys (a multiple of 32)
     int32_t dtype, phase;
     float scale;
     int32_t pad;

@@ -196,6 +196,41 @@ def test_decode_attention_against_float64(dt, b, hq, hkv, t):
     assert float(err.max()) <= tol, float(err.max())
 
 
+@pytest.mark.parametrize("dt", ["fp16", "bf16"])
+@pytest.mark.parametrize("b,hq,hkv,t,sharp", [
+    (1, 1, 1, 1, 1),         # one key
+    (1, 2, 1, 16, 1),        # one block
+    (2, 4, 1, 17, 1),        # one key over
+    (3, 8, 1, 255, 8),       # a block for every warp but a key, peaked scores
+    (16, 32, 32, 5, 1),      # more heads than runs: several heads per run
+    (7, 24, 24, 100, 1),     # runs that end inside a head, 168 heads of 7 blocks
+    (1, 8, 1, 4099, 30),     # one head over many runs, one key dominating
+    (2, 16, 4, 700, 1),
+])
+def test_decode_attention_blocks_and_runs(dt, b, hq, hkv, t, sharp):
+    """Edges of the 16-key blocks and of their runs. Bound per element: the scores' rounding (131 fp32 operations) in the
+    exponent, the exponential, the two-part probabilities (2^-17 bf16, 2^-21 fp16) and the sums, then one rounding."""
+    rng = np.random.default_rng(54)
+    q = O.to_storage((sharp * rng.normal(0, 1, (b, hq, 1, 128))).astype(np.float32), dt)
+    k, v = (O.to_storage(rng.normal(0, 1, (b, hkv, t, 128)).astype(np.float32), dt) for _ in range(2))
+    scale = 1.0 / np.sqrt(128.0)
+    ark.init()
+    tq, tk, tv = (ark.tensor(list(a.shape), NAME[dt]) for a in (q, k, v))
+    out = ark.decode_attention(tq, tk, tv, scale)
+    (got,) = execute([out], {tq: q, tk: k, tv: v})
+    qf, kf, vf = (O.to_f32(x, dt).astype(np.float64) for x in (q, k, v))
+    kf, vf = np.repeat(kf, hq // hkv, axis=1), np.repeat(vf, hq // hkv, axis=1)
+    s = np.einsum("bhqd,bhtd->bhqt", qf, kf) * scale
+    p = np.exp(s - s.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    want = np.einsum("bhqt,bhtd->bhqd", p, vf)
+    one = 2.0 ** -24
+    in_exponent = 131 * one * np.einsum("bhqd,bhtd->bhqt", np.abs(qf), np.abs(kf)).max(-1, keepdims=True) * scale
+    rel = 4 * in_exponent + (t + 64) * one + {"fp16": 2.0 ** -21, "bf16": 2.0 ** -17}[dt]
+    bound = rel * np.einsum("bhqt,bhtd->bhqd", p, np.abs(vf)) + {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want) + 2.0 ** -25
+    assert (np.abs(O.to_f32(got, dt) - want) <= bound).all()
+
+
 @pytest.mark.parametrize("dt,b,hq,hkv,tq,tkv,causal,token_major", [
     ("fp16", 1, 4, 4, 256, 256, True, False),     # two tiles, every head its own K/V
     ("bf16", 2, 8, 2, 384, 384, True, True),      # grouped-query heads, [B, T, H, 128] storage

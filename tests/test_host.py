@@ -507,3 +507,27 @@ def test_bootstrap_allgather_over_gloo_world_size_2(tmp_path):
     outs = [p.communicate(timeout=240)[0] for p in procs]
     for p, o in zip(procs, outs):
         assert p.returncode == 0, o
+
+
+def _stages(build):
+    ark.init()
+    build()
+    from ark_b200.executor import plan_dump
+    return plan_dump(str(ark.Planner(0).plan()))
+
+
+@pytest.mark.parametrize("name,build,chained", [
+    ("tensor and row operands", lambda t: ark.rmsnorm(ark.mul(ark.add(t(64, 512), t(64, 512)), t(1, 512))), True),
+    ("either side of a binary operator", lambda t: ark.softmax(ark.sub(t(64, 512), ark.relu(t(64, 512)))), True),
+    ("in place", lambda t: (lambda x: ark.softmax(ark.add(x, 1.0, x)))(t(64, 512)), True),
+    ("rows that are no whole vectors", lambda t: ark.relu(ark.mul(t(64, 508), t(1, 508))), False),
+    ("longer than the registers of a CTA", lambda t: ark.softmax(ark.add(t(4, 40960), t(4, 40960))), False),
+    ("a column operand", lambda t: ark.rmsnorm(ark.add(t(64, 512), t(64, 1))), False),
+    ("another operator's result", lambda t: (ark.relu(t(64, 512)), ark.softmax(t(64, 512))), False),
+    ("a copy keeps its bits", lambda t: ark.softmax(ark.copy(t(64, 512))), False),
+    ("a masked softmax", lambda t: ark.softmax(ark.add(t(64, 512), t(64, 512)), mask=t(1, 1, 64, 512)), False),
+    ("a row operand that the chain writes", lambda t: (lambda x: ark.add(ark.relu(x, x), ark.sharding(x, 0, 1)[3]))(t(64, 512)), False),
+])
+def test_row_chain_is_formed_only_where_it_is_sound(name, build, chained):
+    text = _stages(lambda: build(lambda *shape: ark.tensor(list(shape), ark.fp16)))
+    assert ("Row chain" in text) == chained, text

@@ -204,6 +204,19 @@ __device__ __forceinline__ void store_vec(T *p, const float (&f)[N]) {
     }
 }
 
+// 32 bytes (a whole sector) per lane and instruction; the address must be a multiple of 32.
+__device__ __forceinline__ void ldg32(const void *p, uint4 &a, uint4 &b) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void stg32(void *p, const uint4 &a, const uint4 &b) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y),
+                 "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+
 // Eight 16-bit elements held in one 16-byte register quad, widened to fp32.
 template <typename T>
 __device__ __forceinline__ void unpack8(const uint4 &q, float (&f)[8]) {

@@ -50,6 +50,33 @@ struct GemmLocal {
     int peer_rows;
 };
 
+// 16 results of a row: whole sectors where the row allows it (half a sector per lane and instruction left the store path at
+// half of its rate).
+template <typename T>
+__device__ __forceinline__ void gemm_store16(T *p, const float *f, bool wide) {
+    union { uint4 q[2]; T e[16]; } o;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) o.e[i] = from_f32<T>(f[i]);
+    if (wide) {
+        stg32(p, o.q[0], o.q[1]);
+    } else {
+        reinterpret_cast<uint4 *>(p)[0] = o.q[0];
+        reinterpret_cast<uint4 *>(p)[1] = o.q[1];
+    }
+}
+template <typename T>
+__device__ __forceinline__ void gemm_load16(const T *p, float (&f)[16], bool wide) {
+    union { uint4 q[2]; T e[16]; } o;
+    if (wide) {
+        ldg32(p, o.q[0], o.q[1]);
+    } else {
+        o.q[0] = ldg16_stream(p);
+        o.q[1] = ldg16_stream(p + 8);
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) f[i] = to_f32(o.e[i]);
+}
+
 template <typename T>
 __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, const T *brow, int col, int ncols,
                                                uint32_t (&r)[32], int cnt, int bcol0 = 0) {
@@ -58,6 +85,7 @@ __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, cons
 #pragma unroll
     for (int i = 0; i < 32; ++i) f[i] = (i < cnt) ? __uint_as_float(r[i]) : 0.0f;
     const bool full = (col + cnt <= ncols) && g.c_vec;
+    const bool wide = (reinterpret_cast<uintptr_t>(crow + col) & 31) == 0;
     if (g.bias_mul == 2) {
         // rotary embedding on the accumulator: brow is the table row of this output row, bcol0 the absolute column of
         // column 0 of `crow` (even; the table row length is a multiple of 8, so an 8-vector never wraps)
@@ -75,15 +103,8 @@ __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, cons
             }
         }
         if (full) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                if (v * 8 < cnt) {
-                    float o[8];
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) o[i] = f[v * 8 + i];
-                    store_vec<T, 8>(crow + col + v * 8, o);
-                }
-            }
+            gemm_store16<T>(crow + col, f, wide);
+            if (cnt == 32) gemm_store16<T>(crow + col + 16, f + 16, wide);
         } else {
 #pragma unroll
             for (int i = 0; i < 32; ++i)
@@ -92,16 +113,15 @@ __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, cons
         return;
     }
     if (full) {
+        float b[2][16];
+        if (brow) {
+            const bool bwide = (reinterpret_cast<uintptr_t>(brow + col) & 31) == 0;
+            gemm_load16<T>(brow + col, b[0], bwide);
+            if (cnt == 32) gemm_load16<T>(brow + col + 16, b[1], bwide);
+        }
         if (brow && !g.bias_mul) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                if (v * 8 < cnt) {
-                    float b[8];
-                    load_vec<T, 8>(brow + col + v * 8, b);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) f[v * 8 + i] += b[i];
-                }
-            }
+            for (int i = 0; i < 32; ++i) f[i] += b[i / 16][i % 16];
         }
         if (g.act != ACT_NONE) {
 #pragma unroll
@@ -109,24 +129,10 @@ __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, cons
         }
         if (brow && g.bias_mul) {
 #pragma unroll
-            for (int v = 0; v < 4; ++v) {
-                if (v * 8 < cnt) {
-                    float b[8];
-                    load_vec<T, 8>(brow + col + v * 8, b);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) f[v * 8 + i] *= b[i];
-                }
-            }
+            for (int i = 0; i < 32; ++i) f[i] *= b[i / 16][i % 16];
         }
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            if (v * 8 < cnt) {
-                float o[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) o[i] = f[v * 8 + i];
-                store_vec<T, 8>(crow + col + v * 8, o);
-            }
-        }
+        gemm_store16<T>(crow + col, f, wide);
+        if (cnt == 32) gemm_store16<T>(crow + col + 16, f + 16, wide);
     } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) {
@@ -148,18 +154,19 @@ __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, cons
 // store of block i. Rows and columns outside the tensor are clipped by TMA.
 template <typename T>
 __device__ __noinline__ void gemm_epilogue_tile_tma(const GemmLocal &g, const CUtensorMap *tmC, const TileCoord &tc, uint32_t tmem_acc,
-                                       int warp, int lane, char *stage, unsigned int &blk, int row_shift = 0) {
+                                       int warp, int lane, char *stage, unsigned int &blk, int grp, int grps, int row_shift = 0) {
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(warp * 32) << 16);
     const int ncols_tile = min(g.tile_n, g.N - tc.n0);
     const int row0 = tc.m0 + warp * 32;
     if (row0 >= g.M) return;  // the whole warp is outside the matrix
-    for (int c = 0; c < g.tile_n; c += 32) {
+    for (int c = grp * 32; c < g.tile_n; c += grps * 32) {
         if (c >= ncols_tile) break;
         uint32_t r[32];
         tmem_ld32(lane_addr + c, r);
-        char *buf = stage + (warp * 2 + (blk & 1)) * kEpiBlockBytes;
-        // the TMA store issued two blocks ago must have finished reading this buffer
-        if (lane == 0) tma_store_wait_read<1>();
+        // one warp per quarter: two buffers each; two warps: one each, and they overlap one another
+        char *buf = stage + (warp * 2 + (grps == 2 ? (unsigned)grp : blk & 1)) * kEpiBlockBytes;
+        // the TMA store that used this buffer last must have finished reading it
+        if (lane == 0) { if (grps == 2) tma_store_wait_read<0>(); else tma_store_wait_read<1>(); }
         __syncwarp();
         tmem_ld_wait();
         union { uint4 q[4]; T e[32]; } o;
@@ -176,7 +183,7 @@ __device__ __noinline__ void gemm_epilogue_tile_tma(const GemmLocal &g, const CU
 }
 
 template <typename T>
-__device__ __noinline__ void gemm_epilogue_tile(const GemmLocal &g, const TileCoord &tc, uint32_t tmem_acc, int warp, int lane) {
+__device__ __noinline__ void gemm_epilogue_tile(const GemmLocal &g, const TileCoord &tc, uint32_t tmem_acc, int warp, int lane, int grp, int grps) {
     const int row = tc.m0 + warp * 32 + lane;
     const bool row_ok = row < g.M;
     const int64_t boff = (int64_t)tc.bn * g.c_stride_n + (int64_t)tc.bc * g.c_stride_c + (int64_t)row * g.ldc;
@@ -185,7 +192,7 @@ __device__ __noinline__ void gemm_epilogue_tile(const GemmLocal &g, const TileCo
     if (g.bias_mul == 2) brow = reinterpret_cast<const T *>(g.bias) + (int64_t)(row_ok ? row % g.rope_rows : 0) * g.rope_cols - tc.n0;
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(warp * 32) << 16);
     const int ncols_tile = min(g.tile_n, g.N - tc.n0);  // valid columns of this tile
-    for (int c = 0; c < g.tile_n; c += 32) {
+    for (int c = grp * 32; c < g.tile_n; c += grps * 32) {
         if (c >= ncols_tile) break;  // uniform across the warp
         uint32_t r[32];
         const int cnt = (g.tile_n - c >= 32) ? 32 : 16;
@@ -201,7 +208,7 @@ __device__ __noinline__ void gemm_epilogue_tile(const GemmLocal &g, const TileCo
 // the 32 lanes of a warp write 32 consecutive n: coalesced without staging.
 // In this form g.M / g.N hold the swapped problem (M' = columns of C, N' = rows of C).
 template <typename T>
-__device__ __noinline__ void gemm_epilogue_tile_swapped(const GemmLocal &g, const TileCoord &tc, uint32_t tmem_acc, int warp, int lane) {
+__device__ __noinline__ void gemm_epilogue_tile_swapped(const GemmLocal &g, const TileCoord &tc, uint32_t tmem_acc, int warp, int lane, int grp, int grps) {
     const int n = tc.m0 + warp * 32 + lane;
     const bool n_ok = n < g.M;
     const int64_t boff = (int64_t)tc.bn * g.c_stride_n + (int64_t)tc.bc * g.c_stride_c;
@@ -209,7 +216,7 @@ __device__ __noinline__ void gemm_epilogue_tile_swapped(const GemmLocal &g, cons
     const T *bbase = g.bias ? reinterpret_cast<const T *>(g.bias) + boff : nullptr;
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(warp * 32) << 16);
     const int rows = min(g.tile_n, g.N - tc.n0);
-    for (int c = 0; c < g.tile_n; c += 32) {
+    for (int c = grp * 32; c < g.tile_n; c += grps * 32) {
         if (c >= rows) break;
         uint32_t r[32];
         const int cnt = (g.tile_n - c >= 32) ? 32 : 16;
@@ -235,7 +242,7 @@ __device__ __noinline__ void gemm_epilogue_tile_swapped(const GemmLocal &g, cons
 // Split-K epilogue of the swapped form: the fp32 partial of k-range `split` goes to
 // ws[split][batch][m][n] unrounded; run_splitk_reduce finishes the job.
 __device__ __noinline__ void gemm_epilogue_tile_partial(const GemmLocal &g, const TileCoord &tc, int split, uint32_t tmem_acc, int warp,
-                                           int lane) {
+                                           int lane, int grp, int grps) {
     const int n = tc.m0 + warp * 32 + lane;   // column of C
     const bool n_ok = n < g.M;                // g.M / g.N hold the swapped problem
     const int64_t ncols = g.M, nrows = g.N;
@@ -243,7 +250,7 @@ __device__ __noinline__ void gemm_epilogue_tile_partial(const GemmLocal &g, cons
     float *w = g.ws + (int64_t)split * g.splits_stride + batch * nrows * ncols;
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(warp * 32) << 16);
     const int rows = min(g.tile_n, (int)nrows - tc.n0);
-    for (int c = 0; c < g.tile_n; c += 32) {
+    for (int c = grp * 32; c < g.tile_n; c += grps * 32) {
         if (c >= rows) break;
         uint32_t r[32];
         const int cnt = (g.tile_n - c >= 32) ? 32 : 16;
@@ -263,14 +270,14 @@ __device__ __noinline__ void gemm_epilogue_tile_partial(const GemmLocal &g, cons
 // Split-K epilogue of the ordinary form: accumulator row = row of C (one per lane), accumulator column = column of C;
 // the fp32 partial of k-range `split` goes to ws[split][batch][m][n] unrounded.
 __device__ __noinline__ void gemm_epilogue_tile_partial_rows(const GemmLocal &g, const TileCoord &tc, int split, uint32_t tmem_acc,
-                                                             int warp, int lane) {
+                                                             int warp, int lane, int grp, int grps) {
     const int m = tc.m0 + warp * 32 + lane;
     const bool m_ok = m < g.M;
     const int64_t batch = (int64_t)tc.bn * g.batch_c + tc.bc;
     float *w = g.ws + (int64_t)split * g.splits_stride + batch * (int64_t)g.M * g.N + (int64_t)m * g.N + tc.n0;
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(warp * 32) << 16);
     const int ncols_tile = min(g.tile_n, g.N - tc.n0);
-    for (int c = 0; c < g.tile_n; c += 32) {
+    for (int c = grp * 32; c < g.tile_n; c += grps * 32) {
         if (c >= ncols_tile) break;
         uint32_t r[32];
         const int cnt = (g.tile_n - c >= 32) ? 32 : 16;
@@ -302,6 +309,9 @@ __device__ __noinline__ void gemm_epilogue_tile_partial_rows(const GemmLocal &g,
 //   credited to the leader's `full` barrier; the leader's commits release the
 //   `empty` slot and publish `acc_full` in both CTAs; the epilogue warps of
 //   both CTAs arrive on the leader's `acc_empty`.
+// Warps per accumulator quarter in the epilogue.
+__device__ __forceinline__ int gemm_epi_groups(int tile_n) { return tile_n > 32 ? 2 : 1; }
+
 // Everything the warp roles of one matmul stage share. Built by every thread at the start of the stage; the roles
 // are separate functions (own register allocation: the threads that issue the copies and the MMAs are the critical
 // path of large matmuls, and spills or extra instructions there cost several per cent).
@@ -520,9 +530,13 @@ __device__ __noinline__ bool gemm_issue(const GemmRun &R) {
     return true;
 }
 
-// Epilogue: warps 0-3, each on its 32-lane quarter of the accumulator.
+// Epilogue: warps 0-3, each on its 32-lane quarter of the accumulator; with tiles of more than 32 columns also warps 8-11,
+// which take every other block of 32 columns of the same quarters: with four warps a tile's epilogue was about 9 us, which
+// bounds products with a short K and shows after the last tile of any (2048 x 11008 x 4096 with SiLU 188 -> 156 us; the
+// 128-token feed-forward block 63.8 -> 61.7 us; whole sectors per store, see gemm_store16, are part of both).
 template <bool PAIR>
-__device__ __noinline__ bool gemm_drain(const GemmRun &R, int warp, int lane) {
+__device__ __noinline__ bool gemm_drain(const GemmRun &R, int warp_id, int lane) {
+    const int warp = warp_id & 3, grp = warp_id >> 3, grps = gemm_epi_groups(R.L.tile_n);
     constexpr bool GROUPED = true;
     const GemmLocal &L = R.L;
     const GemmArgs &g = *R.g;
@@ -566,27 +580,29 @@ __device__ __noinline__ bool gemm_drain(const GemmRun &R, int warp, int lane) {
         tc_fence_after();
         const uint32_t tmem_acc = tmem_base + acc * 256;
         if (L.splits > 1) {
-            if (L.out_transposed) gemm_epilogue_tile_partial(L, tc, split, tmem_acc, warp, lane);
-            else gemm_epilogue_tile_partial_rows(L, tc, split, tmem_acc, warp, lane);
+            if (L.out_transposed) gemm_epilogue_tile_partial(L, tc, split, tmem_acc, warp, lane, grp, grps);
+            else gemm_epilogue_tile_partial_rows(L, tc, split, tmem_acc, warp, lane, grp, grps);
         } else if (L.out_transposed) {
-            if (L.dtype == DT_BF16) gemm_epilogue_tile_swapped<__nv_bfloat16>(L, tc, tmem_acc, warp, lane);
-            else gemm_epilogue_tile_swapped<__half>(L, tc, tmem_acc, warp, lane);
+            if (L.dtype == DT_BF16) gemm_epilogue_tile_swapped<__nv_bfloat16>(L, tc, tmem_acc, warp, lane, grp, grps);
+            else gemm_epilogue_tile_swapped<__half>(L, tc, tmem_acc, warp, lane, grp, grps);
         } else if (L.c_tma) {
             // fused all_reduce: the tile goes to the rank that sums these rows (tiles never straddle two owners)
             const int owner = L.peer_rows > 0 ? tc.m0 / L.peer_rows : 0;
             const CUtensorMap *tm = L.peer_rows > 0 ? &gmaps->tmPeer[owner] : tmC;
             const int shift = owner * L.peer_rows;
-            if (L.dtype == DT_BF16) gemm_epilogue_tile_tma<__nv_bfloat16>(L, tm, tc, tmem_acc, warp, lane, epi_stage, epi_blk, shift);
-            else gemm_epilogue_tile_tma<__half>(L, tm, tc, tmem_acc, warp, lane, epi_stage, epi_blk, shift);
+            if (L.dtype == DT_BF16) gemm_epilogue_tile_tma<__nv_bfloat16>(L, tm, tc, tmem_acc, warp, lane, epi_stage, epi_blk, grp, grps, shift);
+            else gemm_epilogue_tile_tma<__half>(L, tm, tc, tmem_acc, warp, lane, epi_stage, epi_blk, grp, grps, shift);
         } else {
-            if (L.dtype == DT_BF16) gemm_epilogue_tile<__nv_bfloat16>(L, tc, tmem_acc, warp, lane);
-            else gemm_epilogue_tile<__half>(L, tc, tmem_acc, warp, lane);
+            if (L.dtype == DT_BF16) gemm_epilogue_tile<__nv_bfloat16>(L, tc, tmem_acc, warp, lane, grp, grps);
+            else gemm_epilogue_tile<__half>(L, tc, tmem_acc, warp, lane, grp, grps);
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) {
-            if constexpr (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&pp->acc_empty[acc]), 0));
-            else mbar_arrive(&pp->acc_empty[acc]);
+        if (lane == 0) {  // two arrivals per quarter, whether from one warp or from two
+            for (int i = grps; i <= 2; ++i) {
+                if constexpr (PAIR) mbar_arrive_cluster(mapa_u32(smem_u32(&pp->acc_empty[acc]), 0));
+                else mbar_arrive(&pp->acc_empty[acc]);
+            }
         }
     }
     // the stage's output must be in global memory before the CTA reaches the next barrier
@@ -664,7 +680,7 @@ __device__ __noinline__ void run_gemm_t(const GemmArgs &g, const GemmArgs *gmaps
                 gemm_issue<PAIR, GROUPED, false>(R);
             }
         }
-    } else if (warp < kEpiWarps) {
+    } else {
         gemm_drain<PAIR>(R, warp, lane);
     }
     __syncthreads();
@@ -679,17 +695,17 @@ __device__ __noinline__ void run_gemm_t(const GemmArgs &g, const GemmArgs *gmaps
     __syncthreads();
 }
 
-// Warps without a role in the matmul (7..15) do not enter the stage function: its register save area and the
+// Warps without a role in the matmul (7 and 12..15, with narrow tiles 7..15) do not enter the stage function: its register save area and the
 // GemmRun record are ~0.5 KB of local memory per thread, and with 208 KiB of the SM's memory configured as shared
 // there is little L1 left to hold them (an idle pass through the function measured 5.5 us). They only take part in
 // the function's three CTA-wide barriers (and the cluster barrier of a pair).
-__device__ __forceinline__ bool gemm_warp_has_role() {
+__device__ __forceinline__ bool gemm_warp_has_role(int tile_n) {
     const int warp = threadIdx.x >> 5;
-    return warp < kEpiWarps || warp == kProducerWarp || warp == kMmaWarp || warp == kProducerWarpB;
+    return warp < kEpiWarps || (gemm_epi_groups(tile_n) == 2 && warp >= 8 && warp < 8 + kEpiWarps) || warp == kProducerWarp || warp == kMmaWarp || warp == kProducerWarpB;
 }
 __device__ __noinline__ void run_gemm(const GemmArgs &g, const GemmArgs *gmaps, int p, int P, char *smem, GemmPipe *pp, CtaCtl *ctl,
                          DeviceState *st, int stage_idx, unsigned long long spin_limit) {
-    if (!gemm_warp_has_role()) {
+    if (!gemm_warp_has_role(g.tile_n)) {
         __syncthreads();
         __syncthreads();
         __syncthreads();
@@ -700,7 +716,7 @@ __device__ __noinline__ void run_gemm(const GemmArgs &g, const GemmArgs *gmaps, 
 }
 __device__ __noinline__ void run_gemm_pair(const GemmArgs &g, const GemmArgs *gmaps, int p, int P, char *smem, GemmPipe *pp, CtaCtl *ctl,
                               DeviceState *st, int stage_idx, unsigned long long spin_limit) {
-    if (!gemm_warp_has_role()) {
+    if (!gemm_warp_has_role(g.tile_n)) {
         __syncthreads();
         __syncthreads();
         cluster_sync_all();

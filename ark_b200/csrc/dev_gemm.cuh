@@ -252,7 +252,7 @@ __device__ __forceinline__ void gemm_pipe_init(GemmPipe *pp, bool pair) {
     }
     for (int a = 0; a < 2; ++a) {
         mbar_init(&pp->acc_full[a], 1);
-        mbar_init(&pp->acc_empty[a], pair ? 2 * kEpiWarps : kEpiWarps);
+        mbar_init(&pp->acc_empty[a], (pair ? 2 : 1) * 2 * kEpiWarps);  // two arrivals per accumulator quarter
     }
     for (int s = 0; s < kGemmMaxStages; ++s) pp->use[s] = 0;
     pp->tile_count = 0;

@@ -148,6 +148,33 @@ def test_matmul_partial_task_range_follows_plan_tiles():
     assert_matmul_close(got, O.matmul(a, b, "fp16"), "fp16", "partial ranges")
 
 
+@pytest.mark.parametrize("dt", ["fp16", "bf16"])
+@pytest.mark.parametrize("m,n,k", [(129, 16, 64), (130, 48, 128), (257, 264, 192), (300, 1000, 72), (512, 520, 8256)])
+@pytest.mark.parametrize("epilogue", ["silu", "add", "mul"])
+def test_matmul_epilogue_columns_and_sectors(dt, m, n, k, epilogue):
+    """Tiles of one, two and more 32-column blocks for the epilogue's warps; rows that begin on and between 32-byte sectors;
+    long K (stores through shared memory). Bound: the products' fp32 sums, the operator, one rounding."""
+    rng = np.random.default_rng(36)
+    a, b, c = rand(rng, (m, k), dt, -1, 1), rand(rng, (k, n), dt, -1, 1), rand(rng, (m, n), dt, -1, 1)
+    ark.init()
+    ta, tb, tc = (ark.tensor(list(v.shape), NAME[dt]) for v in (a, b, c))
+    with ark.PlannerContext(sync=False):
+        p = ark.matmul(ta, tb)
+        out = ark.silu(p) if epilogue == "silu" else getattr(ark, epilogue)(p, tc)
+    (got,) = execute([out], {ta: a, tb: b, tc: c} if epilogue != "silu" else {ta: a, tb: b})
+    a64, b64, c64 = (O.to_f32(v, dt).astype(np.float64) for v in (a, b, c))
+    prod, off = a64 @ b64, (k + 8) * 2.0 ** -24 * (np.abs(a64) @ np.abs(b64))
+    half_ulp = {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt]
+    off = off + half_ulp * np.abs(prod)  # where the product is stored before the operator reads it
+    if epilogue == "silu":
+        want, bound = prod / (1 + np.exp(-prod)), 1.2 * off + 64 * 2.0 ** -24 * (1 + np.abs(prod)) * np.abs(prod)
+    elif epilogue == "add":
+        want, bound = prod + c64, off
+    else:
+        want, bound = prod * c64, off * np.abs(c64)
+    assert (np.abs(O.to_f32(got, dt) - want) <= bound + half_ulp * (np.abs(want) + bound) + 2.0 ** -25).all()
+
+
 # ---- few activation rows against a weight matrix: the CUDA-core weight-streaming stage ----
 @pytest.mark.parametrize("dt", ["fp16", "bf16"])
 @pytest.mark.parametrize("tb", [True, False])

@@ -4,6 +4,7 @@
 // (ark/api/executor.cpp:226-886, ark/gpu/*).
 #include "executor.hpp"
 
+#include <atomic>
 #include <cuda.h>
 #include <cuda_runtime.h>
 
@@ -276,11 +277,20 @@ size_t Executor::read_stage_times(unsigned long long *out, size_t capacity, int 
 }
 
 void Executor::launch_kernel(int iters) {
-    // barrier counters restart at every launch; iter_total and the status persist
-    CUDA_CHECK(cudaMemsetAsync(state_, 0, sizeof(unsigned long long) * (kMaxSyncGroups + 1), stream_));  // barrier[] and run_seq
+    // a resident kernel starts from zeroed barrier counters, and so does a launch whose predecessors may not have passed all
+    // of their barriers; iter_total and the status persist
+    const bool resident = iters == 0;
+    if (resident || !counters_known_) {
+        CUDA_CHECK(cudaMemsetAsync(state_, 0, sizeof(unsigned long long) * (kMaxSyncGroups + 1), stream_));  // barrier[] and run_seq
+        counter_iters_ = 0;
+    }
     LaunchParams P;
     fill_params(P, iters);
+    P.iter_base = counter_iters_;
+    counters_known_ = false;
     CUDA_CHECK(loop_kernel_launch(P, program_.grid, stream_, program_.smem_bytes));
+    counters_known_ = !resident;
+    counter_iters_ += (unsigned long long)iters;
     ++n_launches_;
 }
 
@@ -349,6 +359,7 @@ void Executor::launch() {
 void Executor::check_status() {
     const int32_t st = *reinterpret_cast<volatile int32_t *>(&host_flags_[1]);
     if (st != ST_OK && st != ST_IDLE_EXIT) {
+        counters_known_ = false;
         arkb_status_snapshot snap = status();
         iters_expected_ = snap.iterations;  // what did run; later requests count from here
         throw Error(E_GPU, "loop kernel gave up: status " + std::to_string(snap.code) + " at stage " +
@@ -382,6 +393,12 @@ void Executor::run(int iter) {
     }
 }
 
+static inline void cpu_relax() {
+#if defined(__x86_64__)
+    __builtin_ia32_pause();
+#endif
+}
+
 void Executor::wait(int64_t max_spin_count) {
     if (!pending_) return;
     CUDA_CHECK(cudaSetDevice(device_id_));
@@ -409,7 +426,16 @@ void Executor::wait(int64_t max_spin_count) {
             relaunch_loop_kernel();
         }
     } else {
-        CUDA_CHECK(cudaStreamSynchronize(stream_));
+        // The kernel writes the count of finished iterations to mapped memory behind its last barrier, when all results are
+        // in memory: seen here before cudaStreamSynchronize would return (with the memset in front of the launch gone, a
+        // 64 x 64 addition takes 13.1 us instead of 17.3). The stream is asked now and then whether the
+        // kernel ended without writing it.
+        volatile unsigned long long *done_iters = reinterpret_cast<volatile unsigned long long *>(&host_flags_[2]);
+        for (int64_t spins = 1; *done_iters != iters_expected_; ++spins) {
+            if ((spins & 0x3fff) == 0 && stream_idle()) break;
+            cpu_relax();
+        }
+        std::atomic_thread_fence(std::memory_order_acquire);
     }
     pending_ = false;
     if (*reinterpret_cast<volatile int32_t *>(&host_flags_[0]) > 0) host_flags_[0] = 0;  // abort path: withdraw the request
@@ -418,6 +444,7 @@ void Executor::wait(int64_t max_spin_count) {
     const unsigned long long done = *reinterpret_cast<volatile unsigned long long *>(&host_flags_[2]);
     if (done != iters_expected_) {
         const unsigned long long want = iters_expected_;
+        counters_known_ = false;
         iters_expected_ = done;
         throw Error(E_GPU, "loop kernel finished " + std::to_string(done) + " iterations, " + std::to_string(want) + " were requested");
     }

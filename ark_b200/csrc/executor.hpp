@@ -80,6 +80,10 @@ class Executor {
     bool compiled_ = false, launched_ = false, stopped_ = false, destroyed_ = false, pending_ = false;
     bool kernel_live_ = false;
     float elapsed_ms_ = -1;
+    // One launch per run: the barrier counters go on from launch to launch (no memset in front of the kernel) as long as
+    // every launch before finished; `counter_iters_` iterations since they were zero.
+    bool counters_known_ = false;
+    unsigned long long counter_iters_ = 0;
     int n_launches_ = 0;
     unsigned long long spin_limit_ = 0, idle_limit_ = 0;
     // Kernel launches that only return when the kernel has ended (CUDA_LAUNCH_BLOCKING, a profiler): a resident

@@ -24,8 +24,8 @@ __device__ __forceinline__ bool in_range(const Stage &S, int cta, int &p, int &P
     return true;
 }
 
-// One pass over the stage list. iter_local counts iterations since this
-// launch (barrier phases); iter_no is the 1-based iteration number over the
+// One pass over the stage list. iter_local counts iterations since
+// the barrier counters were zero (barrier phases); iter_no is the 1-based iteration number over the
 // executor's life (cross-rank epochs and channel flags).
 // Stage records are read through a two-slot cache in shared memory: while a CTA works on stage s the
 // record of stage s+1 (of stage 0 after the last one) is copied asynchronously into the other slot, so
@@ -165,9 +165,9 @@ __device__ __forceinline__ void loop_main(const LaunchParams &P) {
 
     DeviceState *st = P.state;
     const int whole = kMaxSyncGroups - 1;  // barrier counter reserved for the run protocol
-    unsigned long long whole_k = 0;        // whole-grid barriers passed since launch
+    unsigned long long whole_k = P.iter_base;  // whole-grid barriers passed since the counters were zero
     unsigned long long run_seq = 0;        // run requests seen since launch
-    unsigned long long iter_local = 0;
+    unsigned long long iter_local = P.iter_base;
     unsigned long long iter_no = st->iter_total;  // stable: only advanced after the last barrier of a run
 
     for (;;) {
@@ -227,6 +227,7 @@ __device__ __forceinline__ void loop_main(const LaunchParams &P) {
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             st->t_end = globaltimer();
             st->iter_total = iter_no;
+            __threadfence_system();  // results and the words above before the count that the host waits for
             if (st->host_iters) *st->host_iters = iter_no;  // the host checks this count against what it asked for
             __threadfence_system();
             if (P.loop_mode) *P.run_flag = 0;

@@ -522,6 +522,8 @@ struct LaunchParams {
     int32_t n_stages;
     int32_t loop_mode;            // 1: persistent, wait on run_flag; 0: run `iters` once and return
     int32_t iters;
+    int32_t pad;
+    unsigned long long iter_base; // iterations since the barrier counters were zero
     int32_t rank, nranks;
     int32_t peersyncs_per_iter;
     int32_t pair_mode;            // 1: launched as clusters of 2 CTAs, matmul tiles are 256 rows per CTA pair

@@ -52,6 +52,32 @@ def test_iterations_accumulate(loop_mode):
     assert st["n_launches"] == (1 if loop_mode else 2)
 
 
+@pytest.mark.parametrize("runs", [[1] * 40, [3, 1, 2, 7, 1]])
+def test_barriers_go_on_from_launch_to_launch(runs):
+    """One launch per run: grid barriers count on over launches, with several barriers per iteration and after a run on
+    which nothing waited."""
+    ark.init()
+    x, w = ark.tensor([40, 256], ark.fp16), ark.tensor([256], ark.fp16)
+    y = ark.rmsnorm(ark.add(x, 1.0, x), w)
+    z = ark.reduce_sum(y, axis=0)
+    ex = ark.Executor(0, 0, "t", str(ark.Planner(0).plan()), False)
+    ex.set_wait_limit(3_000_000_000)
+    ex.compile()
+    ex.tensor_from_numpy(x, np.zeros((40, 256), np.float16))
+    ex.tensor_from_numpy(w, np.ones(256, np.float16))
+    ex.launch()
+    for i, n in enumerate(runs):
+        ex.run(n)
+        if i % 3 != 1:
+            ex.wait()
+    ex.wait()
+    got, total, st = ex.tensor_to_numpy(x), ex.tensor_to_numpy(z), ex.status()
+    ex.stop()
+    ex.destroy()
+    assert np.all(got == sum(runs)) and st["iterations"] == sum(runs) and st["n_launches"] == len(runs)
+    assert np.allclose(total.astype(np.float32), 40.0, atol=0.1)  # 40 rows of ones, normalised
+
+
 def test_relaunch_after_stop():
     t, o = build_chain()
     ex = ark.Executor(0, 0, "t", str(ark.Planner(0).plan()), True)

@@ -213,7 +213,7 @@ class Executor:
 
     def stage_times(self):
         """Time stamps of the last finished iteration as an int64 array [n_stages, grid, 2] (GPU nanosecond
-        timer; zeros for CTAs outside a stage's processor range). Call after wait()."""
+        timer; zeros for CTAs outside a stage's processor range or without a share of it). Call after wait()."""
         ns, grid, w = ctypes.c_int(), ctypes.c_int(), ctypes.c_size_t()
         _check(lib().arkb_executor_stage_times(self._h, -1, None, 0, None, ctypes.byref(ns), ctypes.byref(grid)))
         out = np.zeros((ns.value, grid.value, 2), np.uint64)

@@ -2483,12 +2483,19 @@ struct Lowerer {
         c.cur = e.out.ptr;
         return chain_writes(c, o.out, (size_t)n * c.esize);
     }
-    // A later stage that is the same norm of the same rows as an operator of the chain, with nothing in between that
-    // changes its operands or touches its result: the chain stores the result there too. Returns its index or 0.
+    // A later stage that is the same norm of the same rows as an operator of the chain, with nothing in between (the rest of
+    // the chain included: results may replace the rows in place) that changes its operands or touches its result: the
+    // chain stores the result there too. Returns its index or 0.
     size_t equal_norm(const Chain &c, size_t k, size_t after) const {
         const RowChainOp &o = c.a.ops[k];
         if (!c.norm_in[k] || o.kind == RC_SOFTMAX) return 0;
         const auto in = span_of(c.norm_in[k], (size_t)c.nelem * c.esize), w = span_of(o.weight, (size_t)c.cols * (o.weight_f32 ? 4 : c.esize));
+        for (size_t m = k; m < (size_t)c.a.n_ops; ++m) {
+            const RowChainOp &q = c.a.ops[m];
+            const size_t bytes = (size_t)c.nelem * (q.kind == RC_CAST ? dtype_size(q.op) : c.esize);
+            for (const void *p : {(const void *)q.out, (const void *)q.out2, (const void *)q.copy})
+                if (p && (overlap(span_of(p, bytes), in) || (o.weight && overlap(span_of(p, bytes), w)))) return 0;
+        }
         auto is_same = [&](const Stage &s) {
             const RowOpArgs &r = s.ro;
             return s.kind == SK_ROWOP && whole_grid(s) && !r.mask && !r.residual && r.in == c.norm_in[k] && r.weight == o.weight && r.eps == o.scalar &&

@@ -354,3 +354,38 @@ def test_reduce_rows_over_many_segments(rows, cols):
     x64 = x.astype(np.float64)
     assert (np.abs(gs.reshape(-1) - x64.sum(0)) <= rows * 2.0 ** -24 * np.abs(x64).sum(0)).all()
     assert np.array_equal(gm.reshape(-1), x.max(0))
+
+
+@pytest.mark.parametrize("norm", ["rmsnorm", "layernorm"])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_equal_norm_behind_a_row_chain(norm, in_place):
+    """A norm that appears again behind the chain: stored by the chain while its rows stay, computed anew once the chain has
+    updated them in place. Norms of fp16 rows of 512: 514 fp32 operations and one rounding."""
+    rng = np.random.default_rng(74)
+    a, b, w = (O.to_storage(rng.normal(0, 1, s).astype(np.float32), "fp16") for s in ((64, 512), (64, 512), (512,)))
+    m = O.to_storage(rng.normal(0, 0.1, (512, 512)).astype(np.float32), "fp16")
+    ark.init()
+    ta, tb, tw, tm = (ark.tensor(list(v.shape), ark.fp16) for v in (a, b, w, m))
+    make = (lambda x: ark.rmsnorm(x, tw)) if norm == "rmsnorm" else (lambda x: ark.layernorm(x))
+    x = ark.add(ta, tb, ta)
+    n = make(x)
+    y = ark.add(n, tb, x) if in_place else x
+    ark.matmul(n, tm)
+    z = make(y)
+    text = ark.plan_dump(str(ark.Planner(0).plan()))
+    assert "Row chain" in text and ("(+ " in text) != in_place, text
+    feeds = {ta: a, tb: b, tm: m, **({tw: w} if norm == "rmsnorm" else {})}
+    got_n, got_y, got_z = execute([n, y, z], feeds)
+    first = O.binary("add", a, b, "fp16")
+
+    def want(rows):
+        r = O.to_f32(rows, "fp16").astype(np.float64)
+        if norm == "rmsnorm":
+            return r / np.sqrt((r * r).mean(1, keepdims=True) + 1e-5) * O.to_f32(w, "fp16")
+        r = r - r.mean(1, keepdims=True)
+        return r / np.sqrt((r * r).mean(1, keepdims=True) + 1e-5)
+
+    assert np.array_equal(got_y, O.binary("add", got_n, b, "fp16") if in_place else first)
+    for got, rows in ((got_n, first), (got_z, got_y)):
+        ref = want(rows)
+        assert (np.abs(O.to_f32(got, "fp16") - ref) <= 2.0 ** -11 * 1.01 * np.abs(ref) + 514 * 2.0 ** -24 * (1 + np.abs(ref))).all()

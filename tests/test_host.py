@@ -531,3 +531,33 @@ def _stages(build):
 def test_row_chain_is_formed_only_where_it_is_sound(name, build, chained):
     text = _stages(lambda: build(lambda *shape: ark.tensor(list(shape), ark.fp16)))
     assert ("Row chain" in text) == chained, text
+
+
+def _twice_normalised(between, norm):
+    """A norm at the end of a chain's rows, then `between`, a matmul that ends the chain, and the norm of the same rows."""
+    def build(t):
+        x, n, w = t(64, 512), t(512), t(512, 512)
+        y = norm(ark.add(x, t(64, 512), x), n)
+        x = between(x, y, t)
+        ark.matmul(y, w)
+        norm(x, n)
+    return build
+
+
+_RMS = lambda x, w: ark.rmsnorm(x, w)
+_LN = lambda x, w: ark.layernorm(x)
+
+
+@pytest.mark.parametrize("name,between,norm,once", [
+    ("rows as they were", lambda x, y, t: x, _RMS, True),
+    ("rows as they were, layernorm", lambda x, y, t: x, _LN, True),
+    ("another tensor is written", lambda x, y, t: (ark.relu(y), x)[1], _RMS, True),
+    ("the chain updates the rows in place", lambda x, y, t: ark.add(y, t(64, 512), x), _RMS, False),
+    ("the chain updates the rows in place, layernorm", lambda x, y, t: ark.add(y, t(64, 512), x), _LN, False),
+    ("with the rows as second operand", lambda x, y, t: ark.add(y, x, x), _RMS, False),
+    ("two operators behind the norm", lambda x, y, t: ark.relu(ark.mul(y, t(64, 512)), x), _RMS, False),
+    ("a stage behind the chain updates them", lambda x, y, t: ark.copy(t(64, 512), x), _RMS, False),
+])
+def test_equal_norm_is_computed_once_only_while_its_rows_stay(name, between, norm, once):
+    text = _stages(lambda: _twice_normalised(between, norm)(lambda *shape: ark.tensor(list(shape), ark.fp16)))
+    assert "Row chain" in text and ("(+ " in text) == once, text

@@ -2300,8 +2300,8 @@ struct Lowerer {
     }
 
     // ---- row chains -----------------------------------------------------------------------------------
-    // Stages that follow each other over the whole grid with nothing but a barrier in between, each working row by row
-    // on the dense result of the one before, become one SK_ROWCHAIN stage. All results are stored as before; operands
+    // Stages that follow each other over the whole grid with nothing but a barrier in between, before and behind, each working
+    // row by row on the dense result of the one before, become one SK_ROWCHAIN stage. All results are stored as before; operands
     // of the chain and its results must either not overlap or be the same elements (every element is then read and
     // written by one thread, in the operators' order).
     struct Chain {
@@ -2537,7 +2537,10 @@ struct Lowerer {
                 if (!chain_add(t, prog.stages[last + 2])) break;
                 c = t;
                 last += 2;
-                if (chain_split(c)) best = c;  // (without a row width yet, or with rows that do not fit, it cannot end here)
+                // It can end here where a barrier of the whole grid follows (a stage that follows without one relies on a
+                // barrier in front of this member, which falls away), with a row width that is known and fits.
+                const bool closed = last + 1 == prog.stages.size() || (prog.stages[last + 1].kind == SK_SYNC && whole_grid(prog.stages[last + 1]));
+                if (closed && chain_split(c)) best = c;
             }
             if (best.stages < 2) continue;
             last = i + 2 * (size_t)(best.stages - 1);

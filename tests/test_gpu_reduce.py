@@ -1,6 +1,8 @@
 """GPU parity: reductions, fused row operators, transpose and embedding
 (reference tests: ark/ops/ops_reduce_test.cpp, ops_transpose_test.cpp,
 ops_embedding_test.cpp)."""
+import json
+
 import numpy as np
 import pytest
 
@@ -389,3 +391,26 @@ def test_equal_norm_behind_a_row_chain(norm, in_place):
     for got, rows in ((got_n, first), (got_z, got_y)):
         ref = want(rows)
         assert (np.abs(O.to_f32(got, "fp16") - ref) <= 2.0 ** -11 * 1.01 * np.abs(ref) + 514 * 2.0 ** -24 * (1 + np.abs(ref))).all()
+
+
+def test_reader_behind_a_row_operator_in_one_resource_group():
+    """x = a + b, then softmax(x) and the column sums of x as task groups of one resource group, with one barrier in front:
+    the sums read what other processors added."""
+    rng = np.random.default_rng(75)
+    a, b = (O.to_storage(rng.normal(0, 1, (600, 1024)).astype(np.float32), "fp16") for _ in range(2))
+    ark.init()
+    ta, tb = ark.tensor([600, 1024], ark.fp16), ark.tensor([600, 1024], ark.fp16)
+    x = ark.add(ta, tb)
+    p, s = ark.softmax(x), ark.reduce_sum(x, axis=0)
+    plan = json.loads(str(ark.Planner(0).plan()))
+    groups = plan["ProcessorGroups"]
+    groups[1]["ResourceGroups"][0]["TaskGroups"] += groups[2]["ResourceGroups"][0]["TaskGroups"]
+    del groups[2]
+    got_x, got_p, got_s = execute([x, p, s], {ta: a, tb: b}, plan=json.dumps(plan))
+    assert np.array_equal(got_x, O.binary("add", a, b, "fp16"))
+    rows = O.to_f32(got_x, "fp16").astype(np.float64)
+    e = np.exp(rows - rows.max(1, keepdims=True))
+    e /= e.sum(1, keepdims=True)
+    # sums and exponentials in fp32 (1024 and 600 terms, exponents up to 10), one rounding; probabilities below fp16's normal range: half its spacing
+    assert (np.abs(O.to_f32(got_p, "fp16") - e) <= (2.0 ** -11 + 2000 * 2.0 ** -24) * e + 2.0 ** -25).all()
+    assert (np.abs(O.to_f32(got_s, "fp16") - rows.sum(0, keepdims=True)) <= 2.0 ** -11 * np.abs(rows.sum(0)) + 600 * 2.0 ** -24 * np.abs(rows).sum(0)).all()

@@ -561,3 +561,26 @@ _LN = lambda x, w: ark.layernorm(x)
 def test_equal_norm_is_computed_once_only_while_its_rows_stay(name, between, norm, once):
     text = _stages(lambda: _twice_normalised(between, norm)(lambda *shape: ark.tensor(list(shape), ark.fp16)))
     assert "Row chain" in text and ("(+ " in text) == once, text
+
+
+@pytest.mark.parametrize("norm", ["LayerNorm", "Softmax", "RMSNorm"])
+@pytest.mark.parametrize("reader", ["ReduceSum", "Matmul", "LayerNorm"])
+def test_row_chain_keeps_the_barrier_that_the_stage_behind_it_needs(norm, reader):
+    """Task groups of one resource group that do not depend on each other follow without a barrier: a chain that took the
+    first of them in would leave the second one, which reads the same rows, without the barrier in front of it."""
+    ark.init()
+    t = lambda *shape: ark.tensor(list(shape), ark.fp16)
+    x = ark.add(t(64, 512), t(64, 512))
+    {"LayerNorm": ark.layernorm, "Softmax": ark.softmax, "RMSNorm": ark.rmsnorm}[norm](x)
+    {"ReduceSum": lambda: ark.reduce_sum(x, axis=0), "Matmul": lambda: ark.matmul(x, t(512, 512)), "LayerNorm": lambda: ark.layernorm(x)}[reader]()
+    plan = json.loads(str(ark.Planner(0).plan()))
+    groups = plan["ProcessorGroups"]
+    assert len(groups) == 3
+    groups[1]["ResourceGroups"][0]["TaskGroups"] += groups[2]["ResourceGroups"][0]["TaskGroups"]
+    del groups[2]
+    from ark_b200.executor import plan_dump
+    stages = [line for line in plan_dump(json.dumps(plan)).splitlines() if line[:1].isdigit()]
+    sync = [i for i, line in enumerate(stages) if "sync group" in line]
+    first = [i for i, line in enumerate(stages) if " Add" in line]
+    behind = [i for i, line in enumerate(stages) if {"ReduceSum": "ReduceSum", "Matmul": "Matmul", "LayerNorm": "LayerNorm"}[reader] in line][-1]
+    assert first == [0] and any(0 < i < behind for i in sync), stages

@@ -360,6 +360,8 @@ void Executor::check_status() {
     const int32_t st = *reinterpret_cast<volatile int32_t *>(&host_flags_[1]);
     if (st != ST_OK && st != ST_IDLE_EXIT) {
         counters_known_ = false;
+        // processors that gave up wait for their copies in flight: a launch of its own is over when the error is reported
+        if (!loop_mode_) CUDA_CHECK(cudaStreamSynchronize(stream_));
         arkb_status_snapshot snap = status();
         iters_expected_ = snap.iterations;  // what did run; later requests count from here
         throw Error(E_GPU, "loop kernel gave up: status " + std::to_string(snap.code) + " at stage " +
@@ -420,7 +422,7 @@ void Executor::wait(int64_t max_spin_count) {
             if (relaunches++ >= 2) {
                 *flag = 0;
                 pending_ = false;
-                iters_expected_ = *reinterpret_cast<volatile unsigned long long *>(&host_flags_[2]);
+                iters_expected_ = status().iterations;
                 throw Error(E_GPU, "run request was not picked up by the loop kernel (relaunched twice)");
             }
             relaunch_loop_kernel();
@@ -445,7 +447,7 @@ void Executor::wait(int64_t max_spin_count) {
     if (done != iters_expected_) {
         const unsigned long long want = iters_expected_;
         counters_known_ = false;
-        iters_expected_ = done;
+        iters_expected_ = status().iterations;  // a failed iteration counts there, not in `done`
         throw Error(E_GPU, "loop kernel finished " + std::to_string(done) + " iterations, " + std::to_string(want) + " were requested");
     }
 }

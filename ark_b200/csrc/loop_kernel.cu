@@ -228,7 +228,8 @@ __device__ __forceinline__ void loop_main(const LaunchParams &P) {
             st->t_end = globaltimer();
             st->iter_total = iter_no;
             __threadfence_system();  // results and the words above before the count that the host waits for
-            if (st->host_iters) *st->host_iters = iter_no;  // the host checks this count against what it asked for
+            // the host checks this count against what it asked for; an iteration that gave up is missing from it
+            if (st->host_iters) *st->host_iters = iter_no - (ok ? 0 : 1);
             __threadfence_system();
             if (P.loop_mode) *P.run_flag = 0;
         }

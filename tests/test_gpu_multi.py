@@ -48,6 +48,19 @@ def test_peer_wait_runs_out_and_reports(same_device):
     assert p.stdout.count("bounded-wait checks passed") == 2
 
 
+def test_peer_wait_runs_out_in_a_launch_of_its_own():
+    """The same without the resident kernel: wait() sees the iteration count stay short and reports the status once the
+    launch is over."""
+    if _ngpus() < 1:
+        pytest.skip("needs a GPU")
+    env = dict(os.environ, NCCL_NVLS_ENABLE="0", ARKB_SAME_DEVICE="1", ARKB_LOOP_MODE="0")
+    cmd = [sys.executable, "-m", "torch.distributed.run", "--nnodes=1", "--nproc-per-node=2",
+           "--master-addr", "127.0.0.1", "--master-port", "29655", os.path.join(ROOT, "tests", "timeout_worker.py")]
+    p = subprocess.run(cmd, capture_output=True, text=True, timeout=600, env=env)
+    assert p.returncode == 0, p.stdout[-3000:] + p.stderr[-3000:]
+    assert p.stdout.count("bounded-wait checks passed") == 2
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_nvls_all_reduce(world):
     """The large all_reduce through the NVSwitch (multimem.ld_reduce / multimem.st over a multicast-bound arena),

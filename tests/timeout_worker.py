@@ -4,7 +4,8 @@ wait() raises GpuError, and the same GPU then runs another executor. Nothing her
 the only failure is a wait that gives up by itself.
 
 ARKB_SAME_DEVICE=1 puts both ranks on GPU 0 (rank 1 never launches a kernel, so only one kernel is ever
-resident); otherwise rank r uses GPU r and a first step in which both ranks run is checked too."""
+resident); otherwise rank r uses GPU r and a first step in which both ranks run is checked too.
+ARKB_LOOP_MODE=0: one launch per run instead of the resident kernel."""
 import os
 import sys
 import time
@@ -37,7 +38,7 @@ def main():
     ark.send_done(s)
     r = ark.recv(dstbuf, 1 - rank, tag=11)
     res = ark.add(r, 0.0)
-    ex = ark.Executor(dev, 0, "timeout", str(ark.Planner(dev).plan()), True, allgather=ag)
+    ex = ark.Executor(dev, 0, "timeout", str(ark.Planner(dev).plan()), os.environ.get("ARKB_LOOP_MODE", "1") != "0", allgather=ag)
     ex.set_wait_limit(LIMIT_NS)
     ex.compile()
     ex.tensor_from_numpy(src, np.full((4, 1024), rank + 1, np.float16))
@@ -63,6 +64,7 @@ def main():
         st = ex.status()
         assert st["code"] == 3, st  # peer flag wait timed out
         assert "status 3" in msg, msg
+        assert st["iterations"] == (1 if same else 2), st  # the failed one is counted by the device, not reported as done
         assert took < 5.0, took  # the limit, not the 10 s default, ended the wait
         assert 0 <= st["stage"] < st["n_stages"]
         try:

@@ -91,6 +91,7 @@ Executor::Executor(int device_id, void *stream, const std::string &name, const s
     if (stream) {
         stream_ = reinterpret_cast<cudaStream_t>(stream);
         own_stream_ = false;
+        shared_stream_ = true;
     } else {
         CUDA_CHECK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         own_stream_ = true;
@@ -277,10 +278,11 @@ size_t Executor::read_stage_times(unsigned long long *out, size_t capacity, int 
 }
 
 void Executor::launch_kernel(int iters) {
-    // a resident kernel starts from zeroed barrier counters, and so does a launch whose predecessors may not have passed all
-    // of their barriers; iter_total and the status persist
+    // A resident kernel starts from zeroed barrier counters, and so does a launch whose predecessors may not have passed all
+    // of their barriers, and every launch on a stream that others hold (they may capture it and replay the launch, which
+    // this count does not see); iter_total and the status persist.
     const bool resident = iters == 0;
-    if (resident || !counters_known_) {
+    if (resident || shared_stream_ || !counters_known_) {
         CUDA_CHECK(cudaMemsetAsync(state_, 0, sizeof(unsigned long long) * (kMaxSyncGroups + 1), stream_));  // barrier[] and run_seq
         counter_iters_ = 0;
     }
@@ -430,14 +432,19 @@ void Executor::wait(int64_t max_spin_count) {
     } else {
         // The kernel writes the count of finished iterations to mapped memory behind its last barrier, when all results are
         // in memory: seen here before cudaStreamSynchronize would return (with the memset in front of the launch gone, a
-        // 64 x 64 addition takes 13.1 us instead of 17.3). The stream is asked now and then whether the
-        // kernel ended without writing it.
-        volatile unsigned long long *done_iters = reinterpret_cast<volatile unsigned long long *>(&host_flags_[2]);
-        for (int64_t spins = 1; *done_iters != iters_expected_; ++spins) {
-            if ((spins & 0x3fff) == 0 && stream_idle()) break;
-            cpu_relax();
+        // 64 x 64 addition takes 13.1 us instead of 17.3). The kernel has then still to retire, which nobody can observe on a
+        // stream that only the executor knows; where others hold the stream (events behind the run, captures), and where
+        // the count stays short because an iteration failed, wait() returns when the stream has finished.
+        if (shared_stream_) {
+            CUDA_CHECK(cudaStreamSynchronize(stream_));
+        } else {
+            volatile unsigned long long *done_iters = reinterpret_cast<volatile unsigned long long *>(&host_flags_[2]);
+            for (int64_t spins = 1; *done_iters != iters_expected_; ++spins) {
+                if ((spins & 0x3fff) == 0 && stream_idle()) break;
+                cpu_relax();
+            }
+            std::atomic_thread_fence(std::memory_order_acquire);
         }
-        std::atomic_thread_fence(std::memory_order_acquire);
     }
     pending_ = false;
     if (*reinterpret_cast<volatile int32_t *>(&host_flags_[0]) > 0) host_flags_[0] = 0;  // abort path: withdraw the request
@@ -515,6 +522,11 @@ void Executor::destroy() {
     stages_dev_ = arena_ = comm_ = state_ = nullptr;
     host_flags_ = nullptr;
     destroyed_ = true;
+}
+
+void *Executor::stream() {
+    shared_stream_ = true;
+    return stream_;
 }
 
 arkb_status_snapshot Executor::status() {

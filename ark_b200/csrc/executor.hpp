@@ -38,7 +38,7 @@ class Executor {
     uintptr_t tensor_address(const std::string &tensor_json) const;
     void tensor_io(const std::string &tensor_json, void *data, size_t bytes, void *stream, bool is_d2d, bool write);
     arkb_status_snapshot status();
-    void *stream() const { return stream_; }
+    void *stream();  // from now on the caller may observe and use it, see shared_stream_
     const Program &program() const { return program_; }
     void set_spin_limit(unsigned long long v) { spin_limit_ = v; }
     void set_idle_limit(unsigned long long v) { idle_limit_ = v; }
@@ -67,6 +67,7 @@ class Executor {
     int num_sm_ = 0;
     cudaStream_t stream_ = nullptr, copy_stream_ = nullptr;
     bool own_stream_ = false;
+    bool shared_stream_ = false;  // the stream came from the caller or its handle was given out
     cudaEvent_t ev_start_ = nullptr, ev_stop_ = nullptr;
     void *workspace_ = nullptr;  // split-K partials
     unsigned long long *stage_times_ = nullptr;  // per-stage, per-CTA time stamps (diagnostic, off by default)

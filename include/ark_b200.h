@@ -103,7 +103,11 @@ arkb_status arkb_executor_launch(arkb_executor *e);
 arkb_status arkb_executor_run(arkb_executor *e, int iter);
 /* Executor::wait(max_spin_count) (executor.hpp:55); a device-side timeout comes back as ARKB_GPU_ERROR,
  * and so does a request whose iterations did not all run: the count of finished iterations the kernel
- * reports is compared with what was asked for, and a request that met no kernel is served by a relaunch. */
+ * reports is compared with what was asked for, and a request that met no kernel is served by a relaunch.
+ * On return the results are in device memory. Without loop mode, the stream has also finished (an event
+ * recorded behind run() is complete) when it came from the caller or arkb_executor_stream has given it out,
+ * and after every error; on a stream of the executor's own that nobody else knows, the kernel may still
+ * be retiring. */
 arkb_status arkb_executor_wait(arkb_executor *e, int64_t max_spin_count);
 /* Executor::stop(max_spin_count) (executor.hpp:61): returns milliseconds between launch and stop. */
 arkb_status arkb_executor_stop(arkb_executor *e, int64_t max_spin_count, float *elapsed_msec);
@@ -125,7 +129,7 @@ arkb_status arkb_executor_tensor_write(arkb_executor *e, const char *tensor_json
 
 /* Device status block and counters (the reference has no equivalent: its device waits are unbounded). */
 arkb_status arkb_executor_status(arkb_executor *e, arkb_run_status *out);
-/* Stream the executor launches on (for callers that record their own events). */
+/* Stream the executor launches on (for callers that record their own events; see arkb_executor_wait). */
 arkb_status arkb_executor_stream(arkb_executor *e, void **stream);
 /* Human-readable dump of the lowered stage program (one line per stage). The
  * returned pointer stays valid until the next call on the same executor.

@@ -78,6 +78,34 @@ def test_barriers_go_on_from_launch_to_launch(runs):
     assert np.allclose(total.astype(np.float32), 40.0, atol=0.1)  # 40 rows of ones, normalised
 
 
+@pytest.mark.parametrize("given", ["handle", "callers_stream", "handle_between"])
+def test_event_behind_run_is_complete_after_wait(given):
+    """A stream that others hold has finished when wait() returns, so the usual pair of events around run() can be read."""
+    torch = pytest.importorskip("torch")
+    ark.init()
+    x = ark.tensor([64, 64], ark.fp16)
+    y = ark.add(x, 1.0)
+    mine = torch.cuda.Stream()
+    ex = ark.Executor(0, mine.cuda_stream if given == "callers_stream" else 0, "t", str(ark.Planner(0).plan()), False)
+    ex.compile()
+    ex.launch()
+    if given == "handle_between":
+        for _ in range(3):  # without a memset in front, then with one
+            ex.run(1)
+            ex.wait()
+    stream = mine if given == "callers_stream" else torch.cuda.ExternalStream(ex.stream())
+    for _ in range(300):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record(stream)
+        ex.run(1)
+        e1.record(stream)
+        ex.wait()
+        assert e1.query() and e0.elapsed_time(e1) > 0.0
+    assert np.all(ex.tensor_to_numpy(y) == 1.0)
+    ex.stop()
+    ex.destroy()
+
+
 def test_relaunch_after_stop():
     t, o = build_chain()
     ex = ark.Executor(0, 0, "t", str(ark.Planner(0).plan()), True)

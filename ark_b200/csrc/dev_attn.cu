@@ -26,7 +26,6 @@
 // 57 -> 38 us.
 #include <type_traits>
 
-#include "dev_attn.cuh"
 #include "dev_common.cuh"
 #include "dev_funcs.h"
 
@@ -58,6 +57,11 @@ __device__ __forceinline__ uint4 lds16(uint32_t a) {
     return v;
 }
 
+__device__ __forceinline__ float exp2_fast(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
 template <typename T>
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     if constexpr (std::is_same_v<T, __nv_bfloat16>)
@@ -270,7 +274,7 @@ template <typename T, int G>
 __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, char *smem) {
     constexpr int D = kHeadDim;
     float *qs = reinterpret_cast<float *>(smem);                 // [G][D], already scaled
-    float *ml = qs + G * D;                                      // [G][2]: maximum (log2 units), exp-sum
+    float *ml = qs + G * D;                                      // [G][2]: maximum, exp-sum
     float *sc = ml + 2 * kMaxGroup;                              // [G][chunk_len]
     float *red = sc + (size_t)G * a.chunk_len;                   // [16][G][D]
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -353,7 +357,7 @@ __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, 
             }
             l = warp_sum(l);
             if (lane == 0) {
-                ml[warp * 2] = m * kLog2e;
+                ml[warp * 2] = m;
                 ml[warp * 2 + 1] = l;
             }
         }
@@ -413,6 +417,73 @@ __device__ __noinline__ void attn_chunks(const DecodeAttnArgs &a, int p, int P, 
     }
 }
 
+// Block form: element d of query head g of head `head` = (sequence, K/V head), un-normalised, and the exp-sum it is to be
+// divided by. Maxima are in log2 units.
+__device__ __forceinline__ float merge_pieces(const AttnPieces &pc, const float *ws, int head, int G, int g, int d, float &l) {
+    const int stride = G * 132;  // records are 16-byte aligned
+    int first, n;
+    const float *w0;
+    if (pc.span == pc.blocks) {  // every head has runs of its own
+        first = head * pc.per_span;
+        n = pc.per_span;
+        w0 = ws + (int64_t)first * stride;
+    } else {
+        first = pc.run_of(head * pc.blocks);
+        n = pc.run_of(head * pc.blocks + pc.blocks - 1) - first + 1;
+        w0 = ws + pc.record(first, head) * stride;
+    }
+    // the head opens every run but the first: those records are per_run apart
+    const float *w1 = ws + (int64_t)(first + 1) * pc.per_run * stride;
+    const int64_t step = (int64_t)pc.per_run * stride;
+    float mx = kLowest, o = 0.0f;
+    l = 0.0f;
+    constexpr int B = 4;  // pieces on their way together
+    for (int c0 = 0; c0 < n; c0 += B) {
+        float2 ml[B];
+        float v[B];
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            if (c0 + c >= n) continue;
+            const float *w = c0 + c == 0 ? w0 : w1 + (c0 + c - 1) * step;
+            ml[c] = __ldcg(reinterpret_cast<const float2 *>(w + G * 128 + 2 * g));
+            v[c] = __ldcg(w + g * 128 + d);
+        }
+        float m = mx;
+#pragma unroll
+        for (int c = 0; c < B; ++c)
+            if (c0 + c < n) m = fmaxf(m, ml[c].x);
+        if (c0 > 0) {
+            const float e = exp2_fast(mx - m);
+            l *= e;
+            o *= e;
+        }
+        mx = m;
+#pragma unroll
+        for (int c = 0; c < B; ++c) {
+            if (c0 + c >= n) continue;
+            const float e = exp2_fast(ml[c].x - mx);
+            l += ml[c].y * e;
+            o += v[c] * e;
+        }
+    }
+    return o;
+}
+
+// Chunk form: the same; maxima as they are.
+__device__ __forceinline__ float merge_chunks(const AttnPieces &pc, const float *ws, int head, int G, int g, int d, float &l) {
+    const float *w = ws + (size_t)head * pc.per_span * G * 132;
+    const size_t stride = (size_t)G * 132;
+    float m = kLowest, o = 0.0f;
+    for (int c = 0; c < pc.per_span; ++c) m = fmaxf(m, w[c * stride + G * 128 + 2 * g]);
+    l = 0.0f;
+    for (int c = 0; c < pc.per_span; ++c) {
+        const float f = __expf(w[c * stride + G * 128 + 2 * g] - m);
+        l += w[c * stride + G * 128 + 2 * g + 1] * f;
+        o += w[c * stride + g * 128 + d] * f;
+    }
+    return o;
+}
+
 // Merges the pieces of every (sequence, query head): thread per output element.
 template <typename T>
 __device__ void attn_merge(const DecodeAttnArgs &a, int p, int P) {
@@ -421,9 +492,10 @@ __device__ void attn_merge(const DecodeAttnArgs &a, int p, int P) {
     T *out = reinterpret_cast<T *>(a.out);
     for (int i = p * (int)blockDim.x + threadIdx.x; i < total; i += P * (int)blockDim.x) {
         const int d = i % D, h = i / D % a.Hq, b = i / (D * a.Hq);
-        float l, o[1];
-        merge_pieces<1>(a.pieces, a.ws, b * a.Hkv + h / G, G, h % G, d, l, o);
-        out[(int64_t)b * a.o_stride_b + (int64_t)h * a.o_stride_h + d] = from_f32<T>(o[0] / l);
+        float l, o;
+        if (a.chunk_len > 0) o = merge_chunks(a.pieces, a.ws, b * a.Hkv + h / G, G, h % G, d, l);
+        else o = merge_pieces(a.pieces, a.ws, b * a.Hkv + h / G, G, h % G, d, l);
+        out[(int64_t)b * a.o_stride_b + (int64_t)h * a.o_stride_h + d] = from_f32<T>(o / l);
     }
 }
 

@@ -19,7 +19,6 @@
 // ws[range][m][n] and the split-K sum stage that follows adds them in range
 // order, applies the activation and rounds (deterministic).
 #include "dev_comm.cuh"
-#include "dev_attn.cuh"
 #include "dev_common.cuh"
 #include "dev_funcs.h"
 
@@ -107,7 +106,7 @@ __device__ __forceinline__ void load_x8(const GemvArgs &a, const PushTo &c, int 
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = 0.0f;
         for (int c = 0; c < a.mg_chunks; ++c) {
-            const float e = exp2_fast(w[c * stride + G * 128 + 2 * g] - mx);  // maxima are in log2 units
+            const float e = __expf(w[c * stride + G * 128 + 2 * g] - mx);
             l += w[c * stride + G * 128 + 2 * g + 1] * e;
             const float2 *o = reinterpret_cast<const float2 *>(w + c * stride + g * 128 + d);
 #pragma unroll

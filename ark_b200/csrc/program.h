@@ -226,7 +226,7 @@ struct SplitKReduceArgs {
 // How a decode attention cuts the K/V cache: 16-key blocks, `blocks` per (sequence, K/V head). Every `span` blocks (all of
 // them, or one head's) are cut into `per_span` runs of rlen + 1 (the first `rem`) and rlen blocks; there are `runs` in
 // all, one per processor. The part of a head in a run is a piece; its record (per query head of the group: 128 outputs; then
-// maximum, in log2 units, and exp-sum for each) is number run * per_run + (head - first head of the run).
+// maximum, in log2 units unless in chunks, and exp-sum for each) is number run * per_run + (head - first head of the run).
 struct AttnPieces {
     int32_t blocks, runs, span, per_span, rlen, rem, per_run;
 #ifdef __CUDACC__
@@ -495,7 +495,7 @@ enum StatusCode : int32_t {
 constexpr int kChannels = 64;  // send/recv flag channels per rank pair
 
 struct DeviceState {
-    unsigned long long barrier[kMaxSyncGroups];  // monotonic arrive counters (host zeroes them at launch)
+    unsigned long long barrier[kMaxSyncGroups];  // monotonic arrive counters (zeroed by the host when a launch cannot go on from the one before)
     unsigned long long run_seq;                  // run requests published by CTA 0 since launch (zeroed at launch)
     unsigned long long iter_total;               // iterations completed over the executor's life (never reset)
     int32_t status;                              // StatusCode (first failure wins)

@@ -13,17 +13,16 @@
 //  * The cache is a list of 16-key blocks, (sequence, K/V head) by (sequence, K/V head), cut into runs of equal length,
 //    one per CTA. The pieces of a head (one from each run that holds some of it) are merged afterwards: fp32 output,
 //    maximum and exp-sum per piece.
-//  * Every warp works alone on every 12th block of a run: the scores of 16 keys x 8 heads and the output are 24 small
-//    tensor-core products (mma.sync m16n8k16: with 8 columns of queries there is nothing a larger tile could fill), an
+//  * Every warp works alone on every 12th block of a run: the scores of 16 keys x 8 heads and the output are 32 small
+//    tensor-core products (mma.sync m16n8k16, heads as its 8 columns: there is nothing a larger tile could fill), an
 //    online softmax sits in between, and no warp waits for another one until the piece is complete.
-//  * Probabilities stay at fp32 accuracy: each is the sum of two 16-bit values, its rounding and the remainder, which
-//    take the two row halves of the same product (heads are 8 of the 16 rows). They are scaled by 2^14, which cancels in
-//    the division by their sum, so that fp16 remainders stay clear of the subnormals.
+//  * Probabilities stay fp32 values: each is the sum of three 16-bit ones, see split3, smallest first. (With two parts, 2^-17 of
+//    bf16, ten times as many bf16 outputs were not the nearest value of their type: 0.2 % instead of 0.02 %.) A block's
+//    products are added to the output in fp32 arithmetic: the tensor core cuts off what it adds to an accumulator.
 //  * K and V go through shared memory only as a queue: a lane brings in exactly the 16-byte pieces that it will use as
 //    operand fragments (the head dimension may be permuted alike in K and Q, or in V and the output), a block of K and
 //    one of V ahead.
-// One B200, bf16: 16 sequences of 4096 keys, 64 / 8 heads 202 -> 75 us (3.6 TB/s); 5 sequences of 1337 keys, 32 heads
-// 57 -> 38 us.
+// One B200, bf16: 16 sequences of 4096 keys, 64 / 8 heads 200 -> 74 us (3.6 TB/s); 5 sequences of 4096 keys, 32 heads 85 us.
 #include <type_traits>
 
 #include "dev_common.cuh"
@@ -87,6 +86,32 @@ __device__ __forceinline__ uint32_t pack2(T a, T b) {
 }
 constexpr float kLowest = -3.402823466e+38f;
 constexpr float kLog2e = 1.4426950408889634f;
+
+// Two probabilities as three 16-bit values each, packed in pairs. bf16: the 24 bits of the fp32 value cut into three times
+// eight, exactly. fp16: rounded value, rounded remainder and what is left, 33 bits (of values scaled by 2^14, so that
+// the remainders stay clear of the subnormals; the scale cancels in the division by the sum). bf16 needs no scale and
+// gets none: outputs near the type's largest value would overflow.
+template <typename T>
+constexpr float kScale = std::is_same_v<T, __nv_bfloat16> ? 1.0f : 16384.0f;
+template <typename T>
+__device__ __forceinline__ void split3(float x, float y, uint32_t (&part)[3]) {
+    if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            part[i] = __byte_perm(__float_as_uint(x), __float_as_uint(y), 0x7632);
+            x -= __uint_as_float(__float_as_uint(x) & 0xffff0000u);
+            y -= __uint_as_float(__float_as_uint(y) & 0xffff0000u);
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const T a = from_f32<T>(x), b = from_f32<T>(y);
+            part[i] = pack2<T>(a, b);
+            x -= to_f32(a);
+            y -= to_f32(b);
+        }
+    }
+}
 
 template <typename T>
 __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *smem) {
@@ -158,22 +183,25 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
         uint4 qf[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) qf[i] = *reinterpret_cast<const uint4 *>(qs + g * kHeadDim + i * 32 + t * 8);
-        float o[16][4] = {};                       // [n-tile 8 h + j]: rows g (rounded probabilities) and g + 8 (remainders)
+        float o[8][4] = {};                        // [4 h + r]: elements 64 h + 8 g + 2 r (, + 1) of heads 2 t, 2 t + 1 (, and again)
         float m0 = kLowest, m1 = kLowest, l0 = 0.0f, l1 = 0.0f;  // heads 2 t and 2 t + 1
         for (int i = 0; i < n_mine; ++i) {
             fetch_wait<1>();  // K of block i; V of block i is on its way
-            float c[4] = {}, d[4] = {};
+            float c[4] = {};
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
                 const uint4 x = lds16(ring + k * 1024), y = lds16(ring + k * 1024 + 512);
-                mma16816<T>(c, x.x, y.x, x.y, y.y, qf[k].x, qf[k].y);
-                mma16816<T>(d, x.z, y.z, x.w, y.w, qf[k].z, qf[k].w);
+                float u[4] = {}, v[4] = {};
+                mma16816<T>(u, x.x, y.x, x.y, y.y, qf[k].x, qf[k].y);
+                mma16816<T>(v, x.z, y.z, x.w, y.w, qf[k].z, qf[k].w);
+#pragma unroll
+                for (int e = 0; e < 4; ++e) c[e] += u[e] + v[e];
             }
             fetch_k(i + 1);
             const int key = (kb0 + warp + i * kWarps) * 16 + g;
             const bool in0 = key < a.T, in1 = key + 8 < a.T;
-            const float s0 = in0 ? (c[0] + d[0]) * to_log2 : -INFINITY, s1 = in0 ? (c[1] + d[1]) * to_log2 : -INFINITY;
-            const float s2 = in1 ? (c[2] + d[2]) * to_log2 : -INFINITY, s3 = in1 ? (c[3] + d[3]) * to_log2 : -INFINITY;
+            const float s0 = in0 ? c[0] * to_log2 : -INFINITY, s1 = in0 ? c[1] * to_log2 : -INFINITY;
+            const float s2 = in1 ? c[2] * to_log2 : -INFINITY, s3 = in1 ? c[3] * to_log2 : -INFINITY;
             float x0 = fmaxf(s0, s2), x1 = fmaxf(s1, s3);
 #pragma unroll
             for (int w = 4; w < 32; w *= 2) {
@@ -188,22 +216,29 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
                 l1 *= f1;
                 m0 = x0;
                 m1 = x1;
-                // the output's rows are heads g: their factors are with the lanes whose t is g / 2
-                const float e0 = __shfl_sync(0xffffffffu, f0, g >> 1), e1 = __shfl_sync(0xffffffffu, f1, g >> 1);
-                const float f = g & 1 ? e1 : e0;
 #pragma unroll
-                for (int n = 0; n < 16; ++n)
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) o[n][e] *= f;
+                for (int n = 0; n < 8; ++n) {
+                    o[n][0] *= f0;
+                    o[n][1] *= f1;
+                    o[n][2] *= f0;
+                    o[n][3] *= f1;
+                }
             }
-            const float p0 = exp2_fast(s0 - m0 + 14.0f), p1 = exp2_fast(s1 - m1 + 14.0f);
-            const float p2 = exp2_fast(s2 - m0 + 14.0f), p3 = exp2_fast(s3 - m1 + 14.0f);
+            // the distance to the maximum in one rounding
+            const float p0 = exp2_fast(in0 ? fmaf(c[0], to_log2, -m0) : -INFINITY) * kScale<T>;
+            const float p1 = exp2_fast(in0 ? fmaf(c[1], to_log2, -m1) : -INFINITY) * kScale<T>;
+            const float p2 = exp2_fast(in1 ? fmaf(c[2], to_log2, -m0) : -INFINITY) * kScale<T>;
+            const float p3 = exp2_fast(in1 ? fmaf(c[3], to_log2, -m1) : -INFINITY) * kScale<T>;
             l0 += p0 + p2;
             l1 += p1 + p3;
-            const T h0 = from_f32<T>(p0), h1 = from_f32<T>(p1), h2 = from_f32<T>(p2), h3 = from_f32<T>(p3);
-            const uint32_t a0 = transpose8x8(pack2<T>(h0, h1)), a2 = transpose8x8(pack2<T>(h2, h3));
-            const uint32_t a1 = transpose8x8(pack2<T>(from_f32<T>(p0 - to_f32(h0)), from_f32<T>(p1 - to_f32(h1))));
-            const uint32_t a3 = transpose8x8(pack2<T>(from_f32<T>(p2 - to_f32(h2)), from_f32<T>(p3 - to_f32(h3))));
+            uint32_t lo[3], hi[3];  // parts for keys g and g + 8, turned into columns of heads
+            split3<T>(p0, p1, lo);
+            split3<T>(p2, p3, hi);
+#pragma unroll
+            for (int e = 0; e < 3; ++e) {
+                lo[e] = transpose8x8(lo[e]);
+                hi[e] = transpose8x8(hi[e]);
+            }
             fetch_wait<1>();
             const uint32_t vs = ring + kBlockBytes;
 #pragma unroll
@@ -213,8 +248,13 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
                 const uint32_t r2[4] = {v2.x, v2.y, v2.z, v2.w}, r3[4] = {v3.x, v3.y, v3.z, v3.w};
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    mma16816<T>(o[h * 8 + 2 * r], a0, a1, a2, a3, __byte_perm(r0[r], r1[r], 0x5410), __byte_perm(r2[r], r3[r], 0x5410));
-                    mma16816<T>(o[h * 8 + 2 * r + 1], a0, a1, a2, a3, __byte_perm(r0[r], r1[r], 0x7632), __byte_perm(r2[r], r3[r], 0x7632));
+                    const uint32_t a0 = __byte_perm(r0[r], r1[r], 0x5410), a1 = __byte_perm(r0[r], r1[r], 0x7632);
+                    const uint32_t a2 = __byte_perm(r2[r], r3[r], 0x5410), a3 = __byte_perm(r2[r], r3[r], 0x7632);
+                    float u[4] = {};
+#pragma unroll
+                    for (int e = 2; e >= 0; --e) mma16816<T>(u, a0, a1, a2, a3, lo[e], hi[e]);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) o[h * 4 + r][e] += u[e];
                 }
             }
             fetch_v(i + 1);
@@ -233,19 +273,18 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
             wl[warp * kMaxGroup + 2 * t + 1] = l1;
         }
         named_barrier(1, kWarps * 32);
-        if (g < G) {
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int head_c = 2 * t + c;
+            if (head_c >= G) continue;
             float m = kLowest;
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) m = fmaxf(m, wm[w * kMaxGroup + g]);
-            const float f = exp2_fast(wm[warp * kMaxGroup + g] - m);
-            float *dst = red + (warp * G + g) * kHeadDim + 16 * t;
+            for (int w = 0; w < kWarps; ++w) m = fmaxf(m, wm[w * kMaxGroup + head_c]);
+            const float f = exp2_fast(wm[warp * kMaxGroup + head_c] - m);
+            float4 *dst = reinterpret_cast<float4 *>(red + (warp * G + head_c) * kHeadDim + 8 * g);
 #pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {  // columns 2 t and 2 t + 1 of n-tile j are elements 16 t + j and 16 t + 8 + j of the half
-                    dst[h * 64 + j] = (o[h * 8 + j][0] + o[h * 8 + j][2]) * f;
-                    dst[h * 64 + 8 + j] = (o[h * 8 + j][1] + o[h * 8 + j][3]) * f;
-                }
+            for (int i = 0; i < 4; ++i)  // elements 64 (i / 2) + 8 g + 4 (i % 2) and the three behind it
+                dst[i / 2 * 16 + i % 2] = make_float4(o[2 * i][c] * f, o[2 * i][c + 2] * f, o[2 * i + 1][c] * f, o[2 * i + 1][c + 2] * f);
         }
         named_barrier(1, kWarps * 32);
         float *out = a.ws + a.pieces.record(p, head) * G * (kHeadDim + 4);

@@ -206,10 +206,16 @@ def test_decode_attention_against_float64(dt, b, hq, hkv, t):
     (7, 24, 24, 100, 1),     # runs that end inside a head, 168 heads of 7 blocks
     (1, 8, 1, 4099, 30),     # one head over many runs, one key dominating
     (2, 16, 4, 700, 1),
+    (3, 4, 4, 1, 1),         # three sequences and more: blocks of 16 keys; one key
+    (3, 8, 4, 16, 1),        # one block, two query heads per K/V head
+    (4, 2, 1, 17, 1),        # a block and one key
+    (5, 16, 2, 192, 1),      # as many blocks as warps
+    (3, 4, 1, 193, 30),      # and one key, one key dominating
+    (20, 16, 8, 64, 8),      # more heads than runs, whole blocks
 ])
 def test_decode_attention_blocks_and_runs(dt, b, hq, hkv, t, sharp):
-    """Edges of the 16-key blocks and of their runs. Bound per element: the scores' rounding (131 fp32 operations) in the
-    exponent, the exponential, the two-part probabilities (2^-17 bf16, 2^-21 fp16) and the sums, then one rounding."""
+    """Edges of the chunks (one and two sequences), of the 16-key blocks and of their runs. Bound per element: the scores'
+    rounding (131 fp32 operations) in the exponent, the exponential and the sums, then one rounding."""
     rng = np.random.default_rng(54)
     q = O.to_storage((sharp * rng.normal(0, 1, (b, hq, 1, 128))).astype(np.float32), dt)
     k, v = (O.to_storage(rng.normal(0, 1, (b, hkv, t, 128)).astype(np.float32), dt) for _ in range(2))
@@ -226,9 +232,35 @@ def test_decode_attention_blocks_and_runs(dt, b, hq, hkv, t, sharp):
     want = np.einsum("bhqt,bhtd->bhqd", p, vf)
     one = 2.0 ** -24
     in_exponent = 131 * one * np.einsum("bhqd,bhtd->bhqt", np.abs(qf), np.abs(kf)).max(-1, keepdims=True) * scale
-    rel = 4 * in_exponent + (t + 64) * one + {"fp16": 2.0 ** -21, "bf16": 2.0 ** -17}[dt]
+    rel = 4 * in_exponent + (t + 64) * one
     bound = rel * np.einsum("bhqt,bhtd->bhqd", p, np.abs(vf)) + {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want) + 2.0 ** -25
     assert (np.abs(O.to_f32(got, dt) - want) <= bound).all()
+
+
+@pytest.mark.parametrize("dt", ["fp16", "bf16"])
+@pytest.mark.parametrize("b", [2, 3])
+def test_decode_attention_keeps_fp32_probabilities(dt, b):
+    """Values that nearly cancel show the probabilities' own accuracy. Four keys, scores of at most 4: 8 products of 16 terms
+    and their sums, one rounding of the exponent's argument and ex2 (2 ulp) stay below 2^-21 of a probability, the sums of
+    four products below 2^-22; 16-bit pairs (2^-17 for bf16) do not."""
+    rng = np.random.default_rng(55)
+    heads, t = 8, 4
+    q, k = (O.to_storage((0.5 * rng.normal(0, 1, (b, heads, n, 128))).astype(np.float32), dt) for n in (1, t))
+    scale = 1.0 / np.sqrt(128.0)
+    s = np.einsum("bhqd,bhtd->bht", *(O.to_f32(x, dt).astype(np.float64) for x in (q, k))) * scale
+    p = np.exp(s - s.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    v = np.zeros((b, heads, t, 128))
+    v[:, :, :2] = O.to_f32(O.to_storage(rng.normal(0, 1, (b, heads, 2, 128)).astype(np.float32), dt), dt)
+    for j in (2, 3):  # each key takes away what is left, up to its own rounding
+        v[:, :, j] = O.to_f32(O.to_storage((-np.einsum("bht,bhtd->bhd", p, v) / p[:, :, j, None]).astype(np.float32), dt), dt)
+    ark.init()
+    tq, tk, tv = (ark.tensor(list(a.shape), NAME[dt]) for a in (q, k, v))
+    out = ark.decode_attention(tq, tk, tv, scale)
+    (got,) = execute([out], {tq: q, tk: k, tv: O.to_storage(v.astype(np.float32), dt)})
+    want = np.einsum("bht,bhtd->bhd", p, v)
+    bound = 1.5 * 2.0 ** -21 * np.einsum("bht,bhtd->bhd", p, np.abs(v)) + {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want) + 2.0 ** -25
+    assert (np.abs(O.to_f32(got, dt).reshape(want.shape) - want) <= bound).all()
 
 
 @pytest.mark.parametrize("dt,b,hq,hkv,tq,tkv,causal,token_major", [

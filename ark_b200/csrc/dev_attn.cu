@@ -113,6 +113,46 @@ __device__ __forceinline__ void split3(float x, float y, uint32_t (&part)[3]) {
     }
 }
 
+// A warp's blocks with plain arithmetic, as the chunk form does it: for infinite or NaN operands (the parts of a probability
+// may be zero, and 0 * inf is NaN) and scores or outputs beyond fp32 that scaling q first, or single products, keep inside.
+// Leaves the output of head h in out[h][128], maxima and exp-sums in wm[h] and wl[h].
+template <typename T>
+__device__ __noinline__ void attn_plain_blocks(const DecodeAttnArgs &a, const T *kbase, const T *vbase, const T *qs, int first, int n_mine,
+                                               float *out, float *wm, float *wl) {
+    const int lane = threadIdx.x & 31, G = a.Hq / a.Hkv;
+    for (int h = 0; h < G; ++h) {
+        float q[4], m = kLowest, l = 0.0f, acc[4] = {};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) q[e] = to_f32(qs[h * kHeadDim + lane * 4 + e]) * a.scale;
+        for (int pass = 0; pass < 2; ++pass)  // the maximum; exponentials and output
+            for (int i = 0; i < n_mine; ++i) {
+                const int key0 = (first + i * kWarps) * 16, keys = min(16, a.T - key0);
+                for (int r = 0; r < keys; ++r) {
+                    float k[4], s = 0.0f;
+                    load_vec<T, 4>(kbase + (int64_t)(key0 + r) * a.k_ld + lane * 4, k);
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) s += q[e] * k[e];
+                    s = warp_sum(s);
+                    if (pass == 0) {
+                        m = fmaxf(m, s);
+                    } else {
+                        const float p = __expf(s - m) * kScale<T>;
+                        float v[4];
+                        load_vec<T, 4>(vbase + (int64_t)(key0 + r) * a.v_ld + lane * 4, v);
+                        l += p;
+#pragma unroll
+                        for (int e = 0; e < 4; ++e) acc[e] += p * v[e];
+                    }
+                }
+            }
+        *reinterpret_cast<float4 *>(out + h * kHeadDim + lane * 4) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+        if (lane == 0) {
+            wm[h] = fmaxf(m * kLog2e, kLowest);
+            wl[h] = l;
+        }
+    }
+}
+
 template <typename T>
 __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *smem) {
     T *qs = reinterpret_cast<T *>(smem + kRingBytes);                      // [8][128], rows of absent heads zero
@@ -260,18 +300,40 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
             fetch_v(i + 1);
         }
         fetch_wait<0>();
-        // the warps' pieces become one: common maximum, rescaled sums and outputs
+        float z = l0 * 0.0f + l1 * 0.0f;  // NaN where something is not finite
 #pragma unroll
-        for (int w = 4; w < 32; w *= 2) {
-            l0 += __shfl_xor_sync(0xffffffffu, l0, w);
-            l1 += __shfl_xor_sync(0xffffffffu, l1, w);
+        for (int n = 0; n < 8; ++n)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) z = fmaf(o[n][e], 0.0f, z);
+        if (__any_sync(0xffffffffu, z != z)) {
+            float *mine = reinterpret_cast<float *>(smem + warp * (kDepth * kBlockBytes));  // this warp's queue, empty by now
+            __syncwarp();
+            attn_plain_blocks<T>(a, kbase, vbase, qs, kb0 + warp, n_mine, mine, wm + warp * kMaxGroup, wl + warp * kMaxGroup);
+            __syncwarp();
+#pragma unroll
+            for (int i = 0; i < 8; ++i)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    if (2 * t + c < G) {
+                        const float *src = mine + (2 * t + c) * kHeadDim + i / 4 * 64 + 8 * g + i % 4 * 2;
+                        o[i][c] = src[0];
+                        o[i][c + 2] = src[1];
+                    }
+        } else {
+            // a warp's exp-sums are spread over its lanes
+#pragma unroll
+            for (int w = 4; w < 32; w *= 2) {
+                l0 += __shfl_xor_sync(0xffffffffu, l0, w);
+                l1 += __shfl_xor_sync(0xffffffffu, l1, w);
+            }
+            if (g == 0) {
+                wm[warp * kMaxGroup + 2 * t] = m0;
+                wm[warp * kMaxGroup + 2 * t + 1] = m1;
+                wl[warp * kMaxGroup + 2 * t] = l0;
+                wl[warp * kMaxGroup + 2 * t + 1] = l1;
+            }
         }
-        if (g == 0) {
-            wm[warp * kMaxGroup + 2 * t] = m0;
-            wm[warp * kMaxGroup + 2 * t + 1] = m1;
-            wl[warp * kMaxGroup + 2 * t] = l0;
-            wl[warp * kMaxGroup + 2 * t + 1] = l1;
-        }
+        // the warps' pieces become one: common maximum, rescaled sums and outputs
         named_barrier(1, kWarps * 32);
 #pragma unroll
         for (int c = 0; c < 2; ++c) {

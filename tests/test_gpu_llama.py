@@ -263,6 +263,44 @@ def test_decode_attention_keeps_fp32_probabilities(dt, b):
     assert (np.abs(O.to_f32(got, dt).reshape(want.shape) - want) <= bound).all()
 
 
+@pytest.mark.parametrize("dt", ["fp16", "bf16"])
+@pytest.mark.parametrize("b", [2, 3])
+def test_decode_attention_with_infinite_and_large_values(dt, b):
+    """Infinite values, NaN and (bf16) values and scores near the end of the range come out as float64 arithmetic says, in both
+    forms of the stage; other columns and heads are not touched by them."""
+    rng = np.random.default_rng(56)
+    heads, kv, t = 8, 4, 300
+    q, k, v = (O.to_f32(O.to_storage(rng.normal(0, 1, (b, h, n, 128)).astype(np.float32), dt), dt) for h, n in ((heads, 1), (kv, t), (kv, t)))
+    v[0, 0, 5, 7], v[0, 0, 299, 8] = np.inf, -np.inf
+    v[0, 1, 20, 3], v[0, 1, 200, 3] = np.inf, -np.inf  # inf - inf
+    v[1, 2, 0, 100] = np.nan
+    k[1, 3, 150, :] = 0.0
+    k[1, 3, 150, 0] = -np.inf * np.sign(q[1, 6, 0, 0])  # no weight for query head 6, infinite or none for head 7
+    if dt == "bf16":
+        v[0, 2, 30, 60] = 3e38
+        q[1, 0, 0, 0], k[1, 0, 17, 0] = 3e19, 2e19  # beyond fp32 before the scale, not behind it
+    q, k, v = (O.to_storage(a, dt) for a in (q, k, v))
+    scale = 1.0 / np.sqrt(128.0)
+    ark.init()
+    tq, tk, tv = (ark.tensor(list(a.shape), NAME[dt]) for a in (q, k, v))
+    out = ark.decode_attention(tq, tk, tv, scale)
+    (got,) = execute([out], {tq: q, tk: k, tv: v})
+    qf, kf, vf = (O.to_f32(x, dt).astype(np.float64) for x in (q, k, v))
+    kf, vf = np.repeat(kf, heads // kv, axis=1), np.repeat(vf, heads // kv, axis=1)
+    with np.errstate(all="ignore"):
+        s = np.einsum("bhqd,bhtd->bhqt", qf, kf) * scale
+        p = np.exp(s - s.max(-1, keepdims=True))
+        p /= p.sum(-1, keepdims=True)
+        want = (p[..., None] * vf[:, :, None]).sum(-2)
+        got = O.to_f32(got, dt).astype(np.float64)
+        assert np.array_equal(np.isnan(got), np.isnan(want))
+        inf = np.isinf(want)
+        assert np.array_equal(got[inf], want[inf]) and inf.any()
+        fine = np.isfinite(want)
+        bound = 2.0 ** -16 * (p[..., None] * np.abs(vf[:, :, None])).sum(-2) + {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want) + 2.0 ** -25
+        assert (np.abs(got - want)[fine] <= bound[fine]).all()
+
+
 @pytest.mark.parametrize("dt,b,hq,hkv,tq,tkv,causal,token_major", [
     ("fp16", 1, 4, 4, 256, 256, True, False),     # two tiles, every head its own K/V
     ("bf16", 2, 8, 2, 384, 384, True, True),      # grouped-query heads, [B, T, H, 128] storage

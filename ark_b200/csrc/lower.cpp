@@ -2349,21 +2349,32 @@ struct Lowerer {
         c.cols = cols;
         return true;
     }
-    // Splits rows over warps; false when a row does not fit the registers of a CTA.
+    static constexpr double kChainFill = 0.7;  // of the lanes
+    // Splits rows over warps; false when a row does not fit the registers of a CTA, or the split would leave too much idle.
     bool chain_split(Chain &c) const {
         const int64_t V = 16 / c.esize, P = prog.grid, warps = kThreads / 32;
         if (c.cols <= 0 || c.cols % V || c.nelem % c.cols || c.nelem / c.cols > INT32_MAX) return false;
         const int64_t nv = c.cols / V, rows = c.nelem / c.cols;
         if (nv < 24 && rows > warps * P) return false;  // most lanes would idle through many rows
         int64_t segs = 1, g = 0;
+        auto fill = [](int64_t n, int64_t lanes) { return (double)n / (double)((n + lanes - 1) / lanes * lanes); };
         if (!c.whole_rows)
-            for (int64_t n = 1; n <= nv && !g; ++n)  // segments of one warp, down to one vector per lane while warps are idle
-                if (nv % n == 0 && nv / n <= 32 * 4 && (rows * n >= warps * P || nv / n <= 32)) { segs = n; g = 1; }
+            // Segments of one warp: at most 4 vectors per lane; down to one while warps are idle. (Many segments of one vector
+            // per lane have too few bytes on their way: embedding and add on 4096 x 520 fp32 13 us in two stages, 18 as a chain
+            // of 26-vector segments.)
+            for (int64_t n = std::min<int64_t>(nv, 32 * 4); n > 0 && !g; --n) {
+                const bool few = rows * (nv / n) < warps * P;
+                if (nv % n == 0 && (n > 32 ? !few : n == nv || rows * (nv / n) < 2 * warps * P) && (fill(n, 32) >= kChainFill || n == nv)) { segs = nv / n; g = 1; }
+            }
         if (!g) {
             for (g = 1; g <= warps && nv > 32 * 4 * g; g *= 2) {}  // 4 vectors per lane leave room for a second operand
             if (g > warps) g = warps;
             if (nv > 32 * 8 * g) return false;
             while (g < warps && rows * g < warps * P && nv > 32 * g) g *= 2;
+            // Elementwise operators alone are better off as stages of their own than with a third of the lanes, or most of the
+            // CTAs, idle: 8192 x 1048 fp32, mul and gelu 60 us in two stages, 70 as a chain of whole rows (262 vectors in 384
+            // lanes), 1024 in segments of two vectors.
+            if (!c.whole_rows && (fill(nv, 32 * g) < kChainFill || rows < P / 4)) return false;
         }
         c.a.warps = (int32_t)g;
         c.a.segs = (int32_t)segs;

@@ -313,7 +313,6 @@ def test_row_chain_leaves_every_result(dt, rows, cols):
     check("s", w["g"] + x, 0)
     check("y", w["s"] / np.sqrt((w["s"] ** 2).mean(1, keepdims=True) + 1e-5) * i["weight"], cols)
     check("d", w["y"] ** 2, 1)
-    assert np.array_equal(got["r"], got["r"])
     check("r", np.maximum(O.to_f32(O.to_storage((w["d"] - 0.5).astype(np.float32), dt), dt), 0), 1, 1 + np.abs(w["d"]))
     z = w["r"] * 0.25
     ez = np.exp(z - z.max(1, keepdims=True))
@@ -322,7 +321,7 @@ def test_row_chain_leaves_every_result(dt, rows, cols):
 
 
 @pytest.mark.parametrize("dt", ["fp32", "fp16", "bf16"])
-@pytest.mark.parametrize("rows,cols", [(7, 320), (9000, 256), (600, 4096)])
+@pytest.mark.parametrize("rows,cols", [(7, 320), (9000, 256), (600, 4096), (3000, 1048), (500, 4168), (3, 8168), (5000, 520)])
 def test_elementwise_row_chain_matches_separate_stages(dt, rows, cols, monkeypatch):
     """Without a reduction the chain may cut rows into segments; the bits are those of the separate stages."""
     rng = np.random.default_rng(72)

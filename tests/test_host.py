@@ -584,3 +584,16 @@ def test_row_chain_keeps_the_barrier_that_the_stage_behind_it_needs(norm, reader
     first = [i for i, line in enumerate(stages) if " Add" in line]
     behind = [i for i, line in enumerate(stages) if {"ReduceSum": "ReduceSum", "Matmul": "Matmul", "LayerNorm": "LayerNorm"}[reader] in line][-1]
     assert first == [0] and any(0 < i < behind for i in sync), stages
+
+
+@pytest.mark.parametrize("cols,segments", [(4096, 4), (1048, 0), (2104, 0), (2136, 3), (4072, 1), (520, 1), (256, 1), (4176, 6)])
+def test_row_chain_segments_keep_the_lanes_busy(cols, segments):
+    """A chain without whole-row operators cuts rows into segments of one warp; a width whose divisors leave many
+    lanes idle stays whole (509 vectors of 8 fp16 values) or in stages of its own (131)."""
+    t = lambda *shape: ark.tensor(list(shape), ark.fp16)
+    text = _stages(lambda: ark.gelu(ark.mul(t(8192, cols), t(1, cols))))
+    found = re.search(r"Row chain rows=8192 cols=(\d+)(?: segments=(\d+))? warps=(\d+)", text)
+    assert (int(found[2] or 1) if found else 0) == segments, text
+    if found:
+        vectors, lanes = int(found[1]) // 8, 32 * int(found[3])
+        assert vectors / (-(-vectors // lanes) * lanes) >= (0.7 if cols > 1024 else 0.5), text

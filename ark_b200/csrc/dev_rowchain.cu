@@ -120,6 +120,9 @@ __device__ __noinline__ void rowchain_typed(const RowChainArgs &a, int p, int P)
             }
         }
         for (int k = 0; k < n_ops; ++k) {
+            // An operand may be an earlier result of the chain, which this thread has just stored: the loads below, which
+            // the compiler takes for reads of no memory, stay behind those stores.
+            asm volatile("" ::: "memory");
             // what the loops below use is copied out of the record: their stores might alias it
             const RowChainOp &o = a.ops[k];
             const int kind = o.kind, op = o.op, mode = o.other_mode;

@@ -572,15 +572,19 @@ __device__ __forceinline__ float merge_pieces(const AttnPieces &pc, const float 
 
 // Chunk form: the same; maxima as they are.
 __device__ __forceinline__ float merge_chunks(const AttnPieces &pc, const float *ws, int head, int G, int g, int d, float &l) {
-    const float *w = ws + (size_t)head * pc.per_span * G * 132;
-    const size_t stride = (size_t)G * 132;
+    const int n = pc.per_span, stride = G * 132;
+    const float *w = ws + (int64_t)head * n * stride, *ml = w + G * 128 + 2 * g;
+    w += g * 128 + d;
     float m = kLowest, o = 0.0f;
-    for (int c = 0; c < pc.per_span; ++c) m = fmaxf(m, w[c * stride + G * 128 + 2 * g]);
+#pragma unroll 4
+    for (int c = 0; c < n; ++c) m = fmaxf(m, __ldcg(ml + c * stride));
     l = 0.0f;
-    for (int c = 0; c < pc.per_span; ++c) {
-        const float f = __expf(w[c * stride + G * 128 + 2 * g] - m);
-        l += w[c * stride + G * 128 + 2 * g + 1] * f;
-        o += w[c * stride + g * 128 + d] * f;
+#pragma unroll 4
+    for (int c = 0; c < n; ++c, w += stride, ml += stride) {
+        const float2 x = __ldcg(reinterpret_cast<const float2 *>(ml));
+        const float v = __ldcg(w), f = __expf(x.x - m);
+        l += x.y * f;
+        o += v * f;
     }
     return o;
 }

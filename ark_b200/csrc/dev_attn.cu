@@ -593,10 +593,11 @@ __device__ __forceinline__ float merge_chunks(const AttnPieces &pc, const float 
 template <typename T>
 __device__ void attn_merge(const DecodeAttnArgs &a, int p, int P) {
     constexpr int D = kHeadDim;
-    const int G = a.Hq / a.Hkv, total = a.B * a.Hq * D;
+    const int G = a.Hq / a.Hkv, rows = a.B * a.Hq;
     T *out = reinterpret_cast<T *>(a.out);
-    for (int i = p * (int)blockDim.x + threadIdx.x; i < total; i += P * (int)blockDim.x) {
-        const int d = i % D, h = i / D % a.Hq, b = i / (D * a.Hq);
+    // a row of 128 outputs per four warps
+    for (int row = p * (kThreads / D) + (int)threadIdx.x / D; row < rows; row += P * (kThreads / D)) {
+        const int d = threadIdx.x % D, h = row % a.Hq, b = row / a.Hq;
         float l, o;
         if (a.chunk_len > 0) o = merge_chunks(a.pieces, a.ws, b * a.Hkv + h / G, G, h % G, d, l);
         else o = merge_pieces(a.pieces, a.ws, b * a.Hkv + h / G, G, h % G, d, l);

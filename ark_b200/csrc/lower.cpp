@@ -1335,13 +1335,18 @@ struct Lowerer {
         a.B = (int32_t)B; a.Hq = (int32_t)Hq; a.Hkv = (int32_t)Hkv; a.T = (int32_t)T;
         a.dtype = q.dtype;
         a.scale = op.has_arg("Scale") ? (float)op.arg_float("Scale") : 1.0f;
-        // 16-key blocks, cut evenly over all processors (a run may then hold the end of one head and the start of the next)
-        // or head by head into as many runs as processors allow. A piece costs about as much as 40 blocks besides its
-        // blocks (start of the stream, sum over the warps: 8 us measured), so 32 heads of 2048 keys are better off with four runs
-        // each on 128 processors, 160 heads of 1337 keys with the even cut.
+        // Two forms. Blocks: 16-key blocks, cut evenly over all processors (a run may then hold the end of one head and the
+        // start of the next) or head by head into as many runs as processors allow. Chunks: a CTA takes chunks of one head.
+        // Microseconds, fitted within 10 % to 3 to 40 sequences of 1 to 4096 keys with 1 to 8 query heads per K/V head (G; the
+        // largest deviations, 20 to 35 %, at G = 8, where the two are a factor apart): blocks 9.3 - 0.25 G, 2.6 + 0.5 G for
+        // each piece of a run and 0.24 for each of its blocks; chunks 8, and for each round 1.45 + 0.85 G and 0.0128 +
+        // 0.0039 G for each key. Many heads of few keys are faster in chunks (8 sequences of 16 keys, 32 heads: 13.7 us
+        // against 21.8), long caches and grouped heads in blocks (16 x 4096, 64 / 8 heads: 75 us against 200). One and two
+        // sequences always take chunks: the weight-streaming matmul behind the attention merges those.
         const int64_t P = proc.count(), nb = (T + 15) / 16, heads = B * Hkv, total = heads * nb;
         if (total > INT32_MAX) throw Error(E_UNSUPPORTED, "DecodeAttention: the cache is too large");
         AttnPieces &pc = a.pieces;
+        const double piece_us = 2.6 + 0.5 * G, block_us = 0.24;
         auto cut = [&](int64_t span, int64_t runs_per_span) {
             pc.blocks = (int32_t)nb;
             pc.span = (int32_t)span;
@@ -1350,36 +1355,48 @@ struct Lowerer {
             pc.rlen = (int32_t)(span / runs_per_span);
             pc.rem = (int32_t)(span % runs_per_span);
             pc.per_run = 1;
-            int64_t most = 0;
+            double most = 0;
             for (int r = 0; r < pc.runs; ++r) {
                 const int64_t b = pc.begin(r), e = r + 1 < pc.runs ? pc.begin(r + 1) : total, pieces = (e - 1) / nb - b / nb + 1;
                 pc.per_run = std::max<int32_t>(pc.per_run, (int32_t)pieces);
-                most = std::max(most, e - b + 40 * pieces);
+                most = std::max(most, block_us * (e - b) + piece_us * pieces);
             }
             return most;
         };
-        if (B <= kGemvMaxM) {
+        double block_form = 1e30;
+        if (B > kGemvMaxM) {
+            AttnPieces best_pc = pc;
+            auto consider = [&](int64_t span, int64_t runs_per_span) {
+                const double c = cut(span, runs_per_span);
+                if (c < block_form) { block_form = c; best_pc = pc; }
+            };
+            consider(total, std::min(P, total));
+            consider(total, std::min<int64_t>(P, (total + 3) / 4));  // fewer pieces to merge
+            if (std::min(nb, P / heads) >= 1) consider(nb, std::min(nb, P / heads));
+            pc = best_pc;
+            block_form += 9.3 - 0.25 * G;
+        }
+        {
             // at most two work items per CTA (one more would cost a third round), at least 128 and at most 2048 keys each;
             // among the candidates the one with the least makespan (rounds x keys per item)
             const int64_t max_chunks = std::max<int64_t>(1, std::min<int64_t>(2 * P / heads, (T + 127) / 128));
-            int64_t best = -1, chunks = 1;
+            int64_t best = -1, chunks = 1, chunk_len = 0, rounds = 0;
             for (int64_t c = 1; c <= max_chunks; ++c) {
                 const int64_t len = std::min<int64_t>(2048, ((T + c - 1) / c + 31) / 32 * 32);
-                const int64_t n = (T + len - 1) / len;
-                const int64_t cost = (heads * n + P - 1) / P * (len + 64);  // 64 keys' worth of fixed cost per item
-                if (best < 0 || cost < best) { best = cost; chunks = n; a.chunk_len = (int32_t)len; }
+                const int64_t n = (T + len - 1) / len, r = (heads * n + P - 1) / P;
+                const int64_t cost = r * (len + 64);  // 64 keys' worth of fixed cost per item
+                if (best < 0 || cost < best) { best = cost; chunks = n; chunk_len = len; rounds = r; }
             }
-            pc.per_span = (int32_t)chunks;
-            pc.rlen = a.chunk_len / 16;
-            pc.blocks = pc.span = pc.per_span * pc.rlen;
-            pc.rem = 0;
-            pc.per_run = 1;
-            pc.runs = (int32_t)(heads * chunks);
-        } else {
-            const int64_t even = std::min<int64_t>(P, (total + 3) / 4);  // at least 4 blocks, more pieces cost more merging
-            const int64_t per_head = std::min(nb, P / heads);
-            const int64_t cost = cut(total, even);
-            if (per_head >= 1 && cut(nb, per_head) > cost) cut(total, even);
+            const double chunk_form = 8.0 + rounds * (1.45 + 0.85 * G + (0.0128 + 0.0039 * G) * chunk_len);
+            if (chunk_form < block_form) {
+                a.chunk_len = (int32_t)chunk_len;
+                pc.per_span = (int32_t)chunks;
+                pc.rlen = a.chunk_len / 16;
+                pc.blocks = pc.span = pc.per_span * pc.rlen;
+                pc.rem = 0;
+                pc.per_run = 1;
+                pc.runs = (int32_t)(heads * chunks);
+            }
         }
         const size_t bytes = (size_t)pc.runs * pc.per_run * G * (128 + 4) * sizeof(float);
         a.ws = env.workspace ? reinterpret_cast<float *>(env.workspace + prog.workspace_bytes) : nullptr;

@@ -206,12 +206,16 @@ def test_decode_attention_against_float64(dt, b, hq, hkv, t):
     (7, 24, 24, 100, 1),     # runs that end inside a head, 168 heads of 7 blocks
     (1, 8, 1, 4099, 30),     # one head over many runs, one key dominating
     (2, 16, 4, 700, 1),
-    (3, 4, 4, 1, 1),         # three sequences and more: blocks of 16 keys; one key
-    (3, 8, 4, 16, 1),        # one block, two query heads per K/V head
-    (4, 2, 1, 17, 1),        # a block and one key
+    (3, 8, 1, 1, 1),         # three sequences and more, in blocks of 16 keys: one key
+    (3, 8, 2, 16, 1),        # one block, four query heads per K/V head
+    (4, 8, 1, 17, 1),        # a block and one key
     (5, 16, 2, 192, 1),      # as many blocks as warps
-    (3, 4, 1, 193, 30),      # and one key, one key dominating
-    (20, 16, 8, 64, 8),      # more heads than runs, whole blocks
+    (3, 8, 1, 193, 30),      # and one key, one key dominating
+    (20, 64, 8, 64, 8),      # more heads than runs, whole blocks
+    (3, 8, 4, 6000, 1),      # two query heads per K/V head
+    (6, 8, 8, 5000, 3),      # one
+    (3, 4, 4, 1, 1),         # heads of few keys, in chunks
+    (40, 8, 4, 33, 1),
 ])
 def test_decode_attention_blocks_and_runs(dt, b, hq, hkv, t, sharp):
     """Edges of the chunks (one and two sequences), of the 16-key blocks and of their runs. Bound per element: the scores'
@@ -235,6 +239,27 @@ def test_decode_attention_blocks_and_runs(dt, b, hq, hkv, t, sharp):
     rel = 4 * in_exponent + (t + 64) * one
     bound = rel * np.einsum("bhqt,bhtd->bhqd", p, np.abs(vf)) + {"fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want) + 2.0 ** -25
     assert (np.abs(O.to_f32(got, dt) - want) <= bound).all()
+
+
+@pytest.mark.parametrize("b,hq,hkv,t", [(2, 4, 2, 100), (4, 16, 2, 100), (5, 4, 4, 100)])
+def test_decode_attention_reads_caches_with_pitches(b, hq, hkv, t):
+    """K and V as parts of larger buffers: rows of 136 and 160 elements, heads and sequences further apart than their rows;
+    chunks and blocks."""
+    rng = np.random.default_rng(57)
+    q, k, v = (O.to_storage(rng.normal(0, 1, (b, h, n, 128)).astype(np.float32), "bf16") for h, n in ((hq, 1), (hkv, t), (hkv, t)))
+    ark.init()
+    tq = ark.tensor(list(q.shape), ark.bf16)
+    tk = ark.tensor(list(k.shape), ark.bf16, strides=[b, hkv + 1, t + 3, 136], padded_shape=list(k.shape))
+    tv = ark.tensor(list(v.shape), ark.bf16, strides=[b, hkv, t + 28, 160], offsets=[0, 0, 16, 32], padded_shape=list(v.shape))
+    out = ark.decode_attention(tq, tk, tv, 0.09)
+    (got,) = execute([out], {tq: q, tk: k, tv: v})
+    qf, kf, vf = (O.to_f32(x, "bf16").astype(np.float64) for x in (q, k, v))
+    kf, vf = np.repeat(kf, hq // hkv, axis=1), np.repeat(vf, hq // hkv, axis=1)
+    s = np.einsum("bhqd,bhtd->bhqt", qf, kf) * 0.09
+    p = np.exp(s - s.max(-1, keepdims=True))
+    p /= p.sum(-1, keepdims=True)
+    want = np.einsum("bhqt,bhtd->bhqd", p, vf)
+    assert (np.abs(O.to_f32(got, "bf16") - want) <= 2.0 ** -16 * np.einsum("bhqt,bhtd->bhqd", p, np.abs(vf)) + 2.0 ** -8 * np.abs(want)).all()
 
 
 @pytest.mark.parametrize("dt", ["fp16", "bf16"])

@@ -597,3 +597,24 @@ def test_row_chain_segments_keep_the_lanes_busy(cols, segments):
     if found:
         vectors, lanes = int(found[1]) // 8, 32 * int(found[3])
         assert vectors / (-(-vectors // lanes) * lanes) >= (0.7 if cols > 1024 else 0.5), text
+
+
+@pytest.mark.parametrize("b,hq,hkv,t,form", [
+    (1, 32, 32, 4096, "chunks"), (2, 64, 8, 4096, "chunks"),            # one and two sequences: merged by the matmul behind
+    (3, 32, 32, 40, "chunks"), (8, 32, 32, 16, "chunks"), (40, 32, 32, 16, "chunks"), (16, 32, 16, 128, "chunks"),
+    (5, 32, 32, 1337, "blocks"), (16, 64, 8, 4096, "blocks"), (8, 64, 8, 40, "blocks"), (16, 32, 32, 1337, "blocks"),
+])
+def test_decode_attention_form_follows_the_shape(b, hq, hkv, t, form):
+    """Many heads of few keys go in chunks, long caches and grouped heads in blocks, as measured."""
+    x = lambda *shape: ark.tensor(list(shape), ark.bf16)
+    text = _stages(lambda: ark.decode_attention(x(b, hq, 1, 128), x(b, hkv, t, 128), x(b, hkv, t, 128), 0.1))
+    assert form + "=" in text, text
+
+
+@pytest.mark.parametrize("b,heads,t", [(3, 96, 1), (5, 40, 16), (7, 8, 1000), (20, 8, 64), (9, 5, 333), (3, 1, 40)])
+def test_decode_attention_runs_cover_the_cache_once(b, heads, t):
+    """The runs of the block form are no more than the processors, and no fewer than leave any idle while blocks are left."""
+    x = lambda *shape: ark.tensor(list(shape), ark.bf16)
+    text = _stages(lambda: ark.decode_attention(x(b, 8 * heads, 1, 128), x(b, heads, t, 128), x(b, heads, t, 128), 0.1))
+    blocks, runs = map(int, re.search(r"blocks=(\d+) runs=(\d+)", text).groups())
+    assert blocks == b * heads * -(-t // 16) and 1 <= runs <= min(148, blocks)

@@ -148,21 +148,33 @@ __device__ __noinline__ void simt_products(const GemmSimtArgs &g, int p, float *
         __syncthreads();
         if (grp == 0) {
             const bool whole = kb1 - kb0 == kblocks;
+            // out of the record: the stores below might alias it (read and tested anew for every result, the activation and
+            // the edges made the stores of a tile 16 us)
+            const int M = g.M, N = g.N, act = g.act, vec = g.vec_c;
+            const int64_t ldc = g.ldc;
             T *C = reinterpret_cast<T *>(g.C) + bn * g.c_stride_n + bc * g.c_stride_c;
             float *piece = g.ws + ((int64_t)p * 2 + (b == b0 ? 0 : 1)) * (TM * TN);
 #pragma unroll
             for (int i = 0; i < 16; ++i) {
                 const float4 o = *reinterpret_cast<const float4 *>(smem + (i * kGroup + t) * 4);
                 const int row = mrow + i / 2, col = ncol + i % 2 * 32;
-                const float v[4] = {acc[i / 2][i % 2 * 4] + o.x, acc[i / 2][i % 2 * 4 + 1] + o.y, acc[i / 2][i % 2 * 4 + 2] + o.z,
+                float v[4] = {acc[i / 2][i % 2 * 4] + o.x, acc[i / 2][i % 2 * 4 + 1] + o.y, acc[i / 2][i % 2 * 4 + 2] + o.z,
                                     acc[i / 2][i % 2 * 4 + 3] + o.w};
                 if (!whole) {
                     *reinterpret_cast<float4 *>(piece + row * TN + col) = make_float4(v[0], v[1], v[2], v[3]);
-                } else if (m0 + row < g.M) {
-                    T *c = C + (int64_t)(m0 + row) * g.ldc + n0 + col;
+                } else if (m0 + row < M && n0 + col < N) {
+                    T *c = C + (int64_t)(m0 + row) * ldc + n0 + col;
+                    if (act != ACT_NONE) {
 #pragma unroll
-                    for (int e = 0; e < 4; ++e)
-                        if (n0 + col + e < g.N) c[e] = from_f32<T>(apply_act(g.act, v[e]));
+                        for (int e = 0; e < 4; ++e) v[e] = apply_act(act, v[e]);
+                    }
+                    if (vec && n0 + col + 4 <= N) {
+                        store_vec<T, 4>(c, v);
+                    } else {
+#pragma unroll
+                        for (int e = 0; e < 4; ++e)
+                            if (n0 + col + e < N) c[e] = from_f32<T>(v[e]);
+                    }
                 }
             }
         }
@@ -201,6 +213,62 @@ __device__ __noinline__ void simt_sums(const GemmSimtArgs &g, int p, int P) {
     }
 }
 
+// Small products: whole 64 x 64 tiles, 2 x 4 results per thread. A tile is a quarter of the other form's, so that few tiles
+// spread over more CTAs, and costs little besides its multiply-adds; see the rule in the lowering.
+template <typename T>
+__device__ __forceinline__ void simt_small(const GemmSimtArgs &g, int p, int P, float *smem) {
+    constexpr int TM = 64, TN = 64, TK = 16;
+    float(*sA)[TM + 1] = reinterpret_cast<float(*)[TM + 1]>(smem);                   // [TK][TM + 1]
+    float(*sB)[TN + 1] = reinterpret_cast<float(*)[TN + 1]>(smem + TK * (TM + 1));   // [TK][TN + 1]
+    const int tiles_m = (g.M + TM - 1) / TM, tiles_n = (g.N + TN - 1) / TN;
+    const int64_t per = (int64_t)tiles_m * tiles_n, total = per * g.batch_c * g.batch_n;
+    const int tid = threadIdx.x, ty = tid / 16, tx = tid % 16;  // rows 2 ty and 2 ty + 1, columns 4 tx to 4 tx + 3
+    for (int64_t u = p; u < total; u += P) {
+        const int batch = (int)(u / per), r = (int)(u % per);
+        const int bc = batch % g.batch_c, bn = batch / g.batch_c;
+        const int m0 = r / tiles_n * TM, n0 = r % tiles_n * TN;
+        const T *A = reinterpret_cast<const T *>(g.A) + bn * g.a_stride_n + bc * g.a_stride_c;
+        const T *B = reinterpret_cast<const T *>(g.B) + bn * g.b_stride_n + bc * g.b_stride_c;
+        T *C = reinterpret_cast<T *>(g.C) + bn * g.c_stride_n + bc * g.c_stride_c;
+        float acc[2][4] = {};
+        for (int k0 = 0; k0 < g.K; k0 += TK) {
+            for (int i = tid; i < TK * TM; i += kThreads) {
+                const int kk = g.trans_a ? i / TM : i % TK, mm = g.trans_a ? i % TM : i / TK;
+                const int m = m0 + mm, k = k0 + kk;
+                float v = 0.0f;
+                if (m < g.M && k < g.K) v = to_f32(g.trans_a ? A[(int64_t)k * g.lda + m] : A[(int64_t)m * g.lda + k]);
+                sA[kk][mm] = v;
+            }
+            for (int i = tid; i < TK * TN; i += kThreads) {
+                const int kk = g.trans_b ? i % TK : i / TN, nn = g.trans_b ? i / TK : i % TN;
+                const int n = n0 + nn, k = k0 + kk;
+                float v = 0.0f;
+                if (n < g.N && k < g.K) v = to_f32(g.trans_b ? B[(int64_t)n * g.ldb + k] : B[(int64_t)k * g.ldb + n]);
+                sB[kk][nn] = v;
+            }
+            __syncthreads();
+#pragma unroll
+            for (int kk = 0; kk < TK; ++kk) {
+                const float a0 = sA[kk][ty * 2], a1 = sA[kk][ty * 2 + 1];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float bv = sB[kk][tx * 4 + j];
+                    acc[0][j] += a0 * bv;
+                    acc[1][j] += a1 * bv;
+                }
+            }
+            __syncthreads();
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int m = m0 + ty * 2 + i, n = n0 + tx * 4 + j;
+                if (m < g.M && n < g.N) C[(int64_t)m * g.ldc + n] = from_f32<T>(apply_act(g.act, acc[i][j]));
+            }
+    }
+}
+
 template <typename T>
 __device__ void simt_typed(const GemmSimtArgs &g, int p, int P, float *smem) {
     if (g.phase == 1) {
@@ -209,6 +277,10 @@ __device__ void simt_typed(const GemmSimtArgs &g, int p, int P, float *smem) {
             case 2: simt_sums<T, 2>(g, p, P); break;
             default: simt_sums<T, 4>(g, p, P); break;
         }
+        return;
+    }
+    if (g.wm == 0) {
+        simt_small<T>(g, p, P, smem);
         return;
     }
     if (p >= g.runs) return;

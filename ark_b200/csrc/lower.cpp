@@ -695,6 +695,19 @@ struct Lowerer {
         const int64_t even = (n + runs - 1) / runs + sum_cost, whole = (tiles + P - 1) / P * g.kblocks;
         if (whole <= even && (tiles <= P || tiles % P == 0)) g.runs = (int32_t)std::min(tiles, P);
         else g.runs = (int32_t)runs;
+        // Small products take whole 64 x 64 tiles: a quarter of the work per tile spreads few tiles over more CTAs, and a tile
+        // costs little besides its multiply-adds. Microseconds, fitted to 1 to 256 products of 1 to 512 rows, 16 to 4096
+        // columns and K of 8 to 1024: small tiles 4 and, for each round, 2.2 + 0.165 K; large ones 12 and, for each
+        // tile of a CTA, 15 + 0.148 K. 512 x 1024 x 64: 16 us small, 31 large; 256 products of 16 x 16 x 16: 11 and
+        // 79; 300 x 1024 x 1024: 175 and 41.
+        const double tiles_each = (double)tiles / g.runs, large = 12 + tiles_each * (15 + 0.148 * (double)g.K);
+        const int64_t small_tiles = ((int64_t)g.M + 63) / 64 * (((int64_t)g.N + 63) / 64) * g.batch_c * g.batch_n;
+        const double small = 4 + (double)((small_tiles + P - 1) / P) * (2.2 + 0.165 * (double)g.K);
+        if (small < large) {
+            g.wm = 0;
+            g.runs = 1;
+            return;
+        }
         g.run_len = (int32_t)(n / g.runs);
         g.run_rem = (int32_t)(n % g.runs);
         const size_t es = dtype_size(g.dtype);
@@ -703,6 +716,7 @@ struct Lowerer {
         };
         g.vec_a = vec(g.A, g.lda, g.a_stride_c, g.a_stride_n);
         g.vec_b = vec(g.B, g.ldb, g.b_stride_c, g.b_stride_n);
+        g.vec_c = vec(g.C, g.ldc, g.c_stride_c, g.c_stride_n);
     }
 
     void lower_matmul(const OpDesc &op, const Range &proc, const TaskGroup &tg, int act, const TensorDesc *act_out,
@@ -757,7 +771,7 @@ struct Lowerer {
             g.trans_a = ta; g.trans_b = tb;
             g.dtype = A.dtype; g.act = act;
             split_simt(g, proc.count());
-            const bool shared = g.kblocks > 1 && simt_tiles(g) % g.runs != 0;
+            const bool shared = g.wm > 0 && g.kblocks > 1 && simt_tiles(g) % g.runs != 0;
             const size_t ws_bytes = shared ? (size_t)g.runs * 2 * kSimtTileElems * sizeof(float) : 0;
             if (shared) {
                 g.ws = reinterpret_cast<float *>(env.workspace + prog.workspace_bytes);
@@ -767,7 +781,7 @@ struct Lowerer {
                 if (simt_tiles(g) > 1) wr(C);  // the tiles that one run holds
             }
             push(s, "Matmul(simt) " + op.name + " M=" + std::to_string(M) + " N=" + std::to_string(N) + " K=" + std::to_string(K) + " tile=" +
-                        std::to_string(32 * g.wm) + "x" + std::to_string(512 / g.wm) + " runs=" + std::to_string(g.runs));
+                        (g.wm == 0 ? std::string("64x64") : std::to_string(32 * g.wm) + "x" + std::to_string(512 / g.wm) + " runs=" + std::to_string(g.runs)));
             if (shared) {
                 GemmSimtArgs sum = g;
                 emit_sync(proc);
@@ -2842,7 +2856,8 @@ struct Lowerer {
                 case SK_PREFILL_ATTN: need = kFullSmemBytes; break;
                 case SK_GEMM_SIMT: {  // two buffers of k-blocks of both operands for each group of threads, every k padded by 4 floats
                     const size_t tk = s.gs.wm == 1 ? 8 : 16;
-                    need = 4 * tk * (size_t)(32 * s.gs.wm + 4 + 512 / s.gs.wm + 4) * sizeof(float) + 1024;
+                    if (s.gs.wm == 0) need = 16 * 1024;
+                    else need = 4 * tk * (size_t)(32 * s.gs.wm + 4 + 512 / s.gs.wm + 4) * sizeof(float) + 1024;
                     break;
                 }
                 case SK_REDUCE: need = (size_t)kThreads * 8 * sizeof(float); break;

@@ -335,11 +335,11 @@ struct GemmSimtArgs {
     int32_t trans_a, trans_b;
     int32_t dtype, act;
     int32_t phase;        // 0: products; 1: adds the pieces of tiles that several runs share (only when there are such tiles)
-    int32_t wm;           // tile: 32 wm rows x 512 / wm columns
+    int32_t wm;           // tile: 32 wm rows x 512 / wm columns; 0: whole 64 x 64 tiles
     int32_t kblocks;      // k-blocks per tile (8 k for wm 1, else 16)
     int32_t runs;         // CTAs the list of all tiles' k-blocks is cut over
     int32_t run_len, run_rem;  // k-blocks of a run; the first run_rem runs have one more
-    int32_t vec_a, vec_b; // 1: base, row pitch and batch strides allow loads of four elements
+    int32_t vec_a, vec_b, vec_c; // 1: base, row pitch and batch strides allow accesses of four elements
     float *ws;            // pieces: [runs][2][tile], a run's first tile in slot 0, a later one in slot 1
 };
 

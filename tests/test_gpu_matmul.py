@@ -106,6 +106,13 @@ def test_matmul_cuda_core_fallback(dt, mnk):
     ("fp32", (148, 64, 40), (40, 128), False, False),           # as many tiles as processors
     ("bf16", (31, 1001), (1001, 259), False, False),
     ("fp16", (70, 333), (129, 333), False, True),
+    ("fp32", (64, 16), (16, 64), False, False),                 # one whole small tile, one k-block
+    ("fp32", (65, 17), (63, 17), False, True),                  # one over, one short
+    ("fp32", (3, 5, 200, 40), (3, 1, 40, 70), False, False),    # small tiles, more than processors, a broadcast operand
+    ("fp32", (50, 130), (50, 129), True, False),                # A transposed, small tiles
+    ("bf16", (5, 9), (9, 67), False, False),
+    ("fp32", (16, 2048), (2048, 513), False, False),            # large 16-row tiles cut into runs, a column over
+    ("fp32", (17, 2047), (2047, 130), False, False),            # rows of results that are no whole vectors
 ])
 def test_matmul_cuda_core_tiles_and_runs(dt, ash, bsh, ta, tb):
     """Edges of the CUDA-core form's three tiles and of its split of the k-blocks over the processors."""
@@ -121,6 +128,24 @@ def test_matmul_cuda_core_tiles_and_runs(dt, ash, bsh, ta, tb):
     # k products summed in fp32 in some order, then one rounding to the storage type
     bound = (a64.shape[-1] + 2) * 2.0 ** -24 * (np.abs(a64) @ np.abs(b64)) + {"fp32": 0, "fp16": 2.0 ** -11, "bf16": 2.0 ** -8}[dt] * np.abs(want)
     assert (np.abs(O.to_f32(got, dt) - want) <= bound + 1e-30).all()
+
+
+@pytest.mark.parametrize("act", ["relu", "gelu", "silu", "sigmoid"])
+@pytest.mark.parametrize("m,n,k", [(40, 70, 24), (300, 262, 700)])  # small tiles; large ones, cut into runs
+def test_matmul_cuda_core_activation(act, m, n, k):
+    rng = np.random.default_rng(36)
+    a, b = rand(rng, (m, k), "fp32", -1.0, 1.0), rand(rng, (k, n), "fp32", -1.0, 1.0)
+    ark.init()
+    t_a, t_b = ark.tensor([m, k], ark.fp32), ark.tensor([k, n], ark.fp32)
+    y = ark.matmul(t_a, t_b)
+    out = {"relu": ark.relu, "gelu": ark.gelu, "silu": lambda x: ark.mul(x, ark.sigmoid(x)), "sigmoid": ark.sigmoid}[act](y)
+    (got,) = execute([out], {t_a: a, t_b: b})
+    x = a.astype(np.float64) @ b
+    want = {"relu": np.maximum(x, 0), "gelu": x / (1 + np.exp(-2 * 0.7978845608028654 * (x + 0.044715 * x ** 3))), "silu": x / (1 + np.exp(-x)),
+            "sigmoid": 1 / (1 + np.exp(-x))}[act]
+    # k products summed in fp32, through activations of slope at most 1.2; their own few roundings relative to the argument
+    bound = 1.2 * (k + 2) * 2.0 ** -24 * (np.abs(a).astype(np.float64) @ np.abs(b)) + 32 * 2.0 ** -24 * (1 + np.abs(x))
+    assert (np.abs(got - want) <= bound).all()
 
 
 def test_matmul_partial_task_range_follows_plan_tiles():

@@ -618,3 +618,11 @@ def test_decode_attention_runs_cover_the_cache_once(b, heads, t):
     text = _stages(lambda: ark.decode_attention(x(b, 8 * heads, 1, 128), x(b, heads, t, 128), x(b, heads, t, 128), 0.1))
     blocks, runs = map(int, re.search(r"blocks=(\d+) runs=(\d+)", text).groups())
     assert blocks == b * heads * -(-t // 16) and 1 <= runs <= min(148, blocks)
+
+
+@pytest.mark.parametrize("a,b,small", [((64, 64), (64, 64), True), ((256, 16, 16), (256, 16, 16), True), ((512, 64), (64, 1024), True),
+                                       ((1, 8), (8, 4096), True), ((300, 4096), (4096, 1024), False), ((1, 4096), (4096, 1024), False),
+                                       ((2048, 2048), (2048, 2048), False), ((64, 256, 512), (64, 512, 256), False)])
+def test_small_full_precision_products_take_small_tiles(a, b, small):
+    text = _stages(lambda: ark.matmul(ark.tensor(list(a), ark.fp32), ark.tensor(list(b), ark.fp32)))
+    assert ("tile=64x64" in text) == small, text

@@ -2846,8 +2846,7 @@ struct Lowerer {
         pair_weight_streams();
         plan_prefetch();
         // dynamic shared memory: the largest need of any stage
-        size_t smem = 16 * 1024;
-        for (auto &s : prog.stages) {
+        auto need_of = [](const Stage &s) {
             size_t need = 0;
             switch (s.kind) {
                 case SK_GEMM:  // ring alone where the epilogue has no staging area
@@ -2880,7 +2879,23 @@ struct Lowerer {
                 }
                 default: break;
             }
-            smem = std::max(smem, need);
+            return need;
+        };
+        // The few-rows ring is short so that the plan leaves shared memory to L1. Where another stage takes more anyway, the ring
+        // has as much (16 rows next to a 2048-row product: 87 us with three slots, 81 with five).
+        auto few_rows = [](const Stage &s) { return s.kind == SK_GEMM && s.gm.out_transposed && s.gm.kgroup > 1 && s.gm.tile_n <= 16; };
+        size_t smem = 16 * 1024;
+        for (auto &s : prog.stages)
+            if (!few_rows(s)) smem = std::max(smem, need_of(s));
+        const size_t ring = std::min<size_t>(std::max<size_t>(smem, kFewRowsRingBytes), kSwappedRingBytes);
+        for (size_t i = 0; i < prog.stages.size(); ++i) {
+            if (!few_rows(prog.stages[i])) continue;
+            GemmArgs &g = prog.stages[i].gm;
+            const std::string was = " stages=" + std::to_string(g.stages) + "x";
+            g.stages = (int32_t)std::min<size_t>(12, ring / (g.kgroup * (16 * 1024 + g.stage_b_bytes)));
+            const size_t at = prog.notes[i].find(was);
+            if (at != std::string::npos) prog.notes[i].replace(at, was.size(), " stages=" + std::to_string(g.stages) + "x");
+            smem = std::max(smem, need_of(prog.stages[i]));
         }
         prog.smem_bytes = std::min<size_t>((smem + 1023) / 1024 * 1024, kFullSmemBytes);
         if (const char *e = getenv("ARKB_FULL_SMEM")) if (atoi(e)) prog.smem_bytes = kFullSmemBytes;

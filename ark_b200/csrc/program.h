@@ -156,9 +156,9 @@ struct RowChainArgs {
 // area (the swapped and split-K forms); stages with a TMA-store epilogue use the first 192 KiB only.
 constexpr int kSwappedRingBytes = 208 * 1024;
 // With at most 16 rows of activations three slots of two k-blocks keep 72 KiB per SM on their way, more than the 53 KiB
-// that HBM's bandwidth and latency ask for, and a plan of such stages leaves half of the SM's memory to L1, where the
-// stage functions' register save areas then stay (five sequences, 7B-shaped, with
-// the attention's queues cut alike: two layers 536 -> 490 us).
+// that HBM's bandwidth and latency ask for, and a plan whose other stages need no more either leaves half of the SM's memory
+// to L1, where the stage functions' register save areas then stay (five sequences, 7B-shaped, with the attention's
+// queues cut alike: two layers 536 -> 490 us of stage time).
 constexpr int kFewRowsRingBytes = 108 * 1024;
 
 struct GemmArgs {

@@ -626,3 +626,13 @@ def test_decode_attention_runs_cover_the_cache_once(b, heads, t):
 def test_small_full_precision_products_take_small_tiles(a, b, small):
     text = _stages(lambda: ark.matmul(ark.tensor(list(a), ark.fp32), ark.tensor(list(b), ark.fp32)))
     assert ("tile=64x64" in text) == small, text
+
+
+def test_ring_of_few_rows_is_short_only_where_the_plan_stays_small():
+    """Three slots next to stages that need as little shared memory, six (a pair of CTAs shares the activations) next to one
+    that takes all of it."""
+    t = lambda *shape: ark.tensor(list(shape), ark.bf16)
+    few = lambda: ark.matmul(t(16, 4096), t(11008, 4096), transpose_other=True)
+    assert re.search(r"M=16 .* stages=3x2kb", _stages(few))
+    both = lambda: (few(), ark.matmul(t(2048, 4096), t(512, 4096), transpose_other=True))
+    assert re.search(r"M=16 .* stages=6x2kb", _stages(both))

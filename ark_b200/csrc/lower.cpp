@@ -148,6 +148,9 @@ struct Lowerer {
         prog.notes.push_back(os.str());
     }
 
+    struct TooManyRanges : Error {
+        TooManyRanges() : Error(E_UNSUPPORTED, "too many distinct processor ranges need a barrier") {}
+    };
     void emit_sync(const Range &r) {
         if (r.count() <= 0) return;
         auto key = std::make_tuple(r.b, r.e, r.s);
@@ -155,7 +158,7 @@ struct Lowerer {
         int id;
         if (it == sync_ids.end()) {
             id = (int)sync_ids.size();
-            if (id >= kMaxSyncGroups - 1) throw Error(E_UNSUPPORTED, "too many distinct processor ranges need a barrier");
+            if (id >= kMaxSyncGroups - 1) throw TooManyRanges();
             sync_ids[key] = id;
         } else {
             id = it->second;
@@ -676,7 +679,10 @@ struct Lowerer {
         const int64_t tm = 32 * g.wm, tn = 512 / g.wm;
         return (g.M + tm - 1) / tm * ((g.N + tn - 1) / tn) * g.batch_c * g.batch_n;
     }
-    static void split_simt(GemmSimtArgs &g, int64_t P) {
+    // A product that is cut into runs needs a barrier of its processors, whose number is limited: a plan that would have too
+    // many with these is lowered again without them.
+    bool cut_simt = true, simt_cut_seen = false;
+    void split_simt(GemmSimtArgs &g, int64_t P) const {
         // The tile with the least padding; flat tiles move more operand bytes per multiply-add, so they are for few rows.
         const double cost[3] = {1.0, 1.05, 1.3};
         double best = 1e300;
@@ -703,7 +709,8 @@ struct Lowerer {
         const double tiles_each = (double)tiles / g.runs, large = 12 + tiles_each * (15 + 0.148 * (double)g.K);
         const int64_t small_tiles = ((int64_t)g.M + 63) / 64 * (((int64_t)g.N + 63) / 64) * g.batch_c * g.batch_n;
         const double small = 4 + (double)((small_tiles + P - 1) / P) * (2.2 + 0.165 * (double)g.K);
-        if (small < large) {
+        const bool cut = g.kblocks > 1 && tiles % g.runs != 0;
+        if (small < large || (cut && !cut_simt)) {
             g.wm = 0;
             g.runs = 1;
             return;
@@ -784,6 +791,7 @@ struct Lowerer {
                         (g.wm == 0 ? std::string("64x64") : std::to_string(32 * g.wm) + "x" + std::to_string(512 / g.wm) + " runs=" + std::to_string(g.runs)));
             if (shared) {
                 GemmSimtArgs sum = g;
+                simt_cut_seen = true;
                 emit_sync(proc);
                 Stage r = new_stage(SK_GEMM_SIMT, proc);
                 r.gs = sum;
@@ -1741,7 +1749,7 @@ struct Lowerer {
         int id;
         if (it == sync_ids.end()) {
             id = (int)sync_ids.size();
-            if (id >= kMaxSyncGroups - 1) throw Error(E_UNSUPPORTED, "too many distinct processor ranges need a barrier");
+            if (id >= kMaxSyncGroups - 1) throw TooManyRanges();
             sync_ids[key] = id;
         } else {
             id = it->second;
@@ -2923,8 +2931,16 @@ std::string Program::dump() const {
 
 Program lower_plan(const Plan &plan, const Layout &lay, const LowerEnv &env) {
     Lowerer lw(plan, lay, env);
-    lw.run();
-    return lw.prog;
+    try {
+        lw.run();
+        return lw.prog;
+    } catch (const Lowerer::TooManyRanges &) {
+        if (!lw.cut_simt || !lw.simt_cut_seen) throw;
+    }
+    Lowerer whole(plan, lay, env);
+    whole.cut_simt = false;
+    whole.run();
+    return whole.prog;
 }
 
 }  // namespace arkb

@@ -636,3 +636,17 @@ def test_ring_of_few_rows_is_short_only_where_the_plan_stays_small():
     assert re.search(r"M=16 .* stages=3x2kb", _stages(few))
     both = lambda: (few(), ark.matmul(t(2048, 4096), t(512, 4096), transpose_other=True))
     assert re.search(r"M=16 .* stages=6x2kb", _stages(both))
+
+
+def test_many_ranges_of_full_precision_products_still_lower():
+    """A product that is cut into runs takes a barrier of its range; the ranges that can have one are limited, and a plan
+    with more of them is lowered with whole tiles instead of being refused."""
+    ark.init()
+    t = lambda *shape: ark.tensor(list(shape), ark.fp32)
+    for i in range(70):
+        with ark.PlannerContext(processor_range=[2 * i, 2 * i + 2]):
+            ark.matmul(t(64, 4096), t(64, 4096), transpose_other=True)
+    from ark_b200.executor import plan_dump
+    plan = str(ark.Planner(0).plan())
+    assert len({tuple(g["ProcessorRange"]) for g in json.loads(plan)["ProcessorGroups"]}) == 70
+    assert plan_dump(plan).count("Matmul(simt)") == 70

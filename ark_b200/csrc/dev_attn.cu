@@ -300,12 +300,20 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
             fetch_v(i + 1);
         }
         fetch_wait<0>();
+#pragma unroll
+        for (int w = 4; w < 32; w *= 2) {  // a warp's exp-sums are spread over its lanes
+            l0 += __shfl_xor_sync(0xffffffffu, l0, w);
+            l1 += __shfl_xor_sync(0xffffffffu, l1, w);
+        }
         float z = l0 * 0.0f + l1 * 0.0f;  // NaN where something is not finite
 #pragma unroll
         for (int n = 0; n < 8; ++n)
 #pragma unroll
             for (int e = 0; e < 4; ++e) z = fmaf(o[n][e], 0.0f, z);
-        if (__any_sync(0xffffffffu, z != z)) {
+        // A sum below the largest score's own 1: all scores are -inf, maybe only before their scale, or so large (2^24) that the
+        // rounding of the maximum takes whole powers of two from every exponential.
+        const bool lost = n_mine > 0 && fminf(l0, l1) < 0.5f * kScale<T>;
+        if (__any_sync(0xffffffffu, z != z || lost)) {
             float *mine = reinterpret_cast<float *>(smem + warp * (kDepth * kBlockBytes));  // this warp's queue, empty by now
             __syncwarp();
             attn_plain_blocks<T>(a, kbase, vbase, qs, kb0 + warp, n_mine, mine, wm + warp * kMaxGroup, wl + warp * kMaxGroup);
@@ -320,12 +328,6 @@ __device__ __noinline__ void attn_pieces(const DecodeAttnArgs &a, int p, char *s
                         o[i][c + 2] = src[1];
                     }
         } else {
-            // a warp's exp-sums are spread over its lanes
-#pragma unroll
-            for (int w = 4; w < 32; w *= 2) {
-                l0 += __shfl_xor_sync(0xffffffffu, l0, w);
-                l1 += __shfl_xor_sync(0xffffffffu, l1, w);
-            }
             if (g == 0) {
                 wm[warp * kMaxGroup + 2 * t] = m0;
                 wm[warp * kMaxGroup + 2 * t + 1] = m1;

@@ -301,6 +301,7 @@ def test_decode_attention_with_infinite_and_large_values(dt, b):
     v[1, 2, 0, 100] = np.nan
     k[1, 3, 150, :] = 0.0
     k[1, 3, 150, 0] = -np.inf * np.sign(q[1, 6, 0, 0])  # no weight for query head 6, infinite or none for head 7
+    q[0, 6, 0, 0], k[0, 3], k[0, 3, :, 0] = (3e19, 0.0, -2e19) if dt == "bf16" else (3e4, 0.0, -2e4)  # every key of a head far below 0
     if dt == "bf16":
         v[0, 2, 30, 60] = 3e38
         q[1, 0, 0, 0], k[1, 0, 17, 0] = 3e19, 2e19  # beyond fp32 before the scale, not behind it

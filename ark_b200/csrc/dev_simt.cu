@@ -147,33 +147,43 @@ __device__ __noinline__ void simt_products(const GemmSimtArgs &g, int p, float *
         }
         __syncthreads();
         if (grp == 0) {
-            const bool whole = kb1 - kb0 == kblocks;
-            // out of the record: the stores below might alias it (read and tested anew for every result, the activation and
-            // the edges made the stores of a tile 16 us)
-            const int M = g.M, N = g.N, act = g.act, vec = g.vec_c;
-            const int64_t ldc = g.ldc;
-            T *C = reinterpret_cast<T *>(g.C) + bn * g.c_stride_n + bc * g.c_stride_c;
-            float *piece = g.ws + ((int64_t)p * 2 + (b == b0 ? 0 : 1)) * (TM * TN);
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
+            auto sums = [&](int i, float (&v)[4]) {
                 const float4 o = *reinterpret_cast<const float4 *>(smem + (i * kGroup + t) * 4);
-                const int row = mrow + i / 2, col = ncol + i % 2 * 32;
-                float v[4] = {acc[i / 2][i % 2 * 4] + o.x, acc[i / 2][i % 2 * 4 + 1] + o.y, acc[i / 2][i % 2 * 4 + 2] + o.z,
-                                    acc[i / 2][i % 2 * 4 + 3] + o.w};
-                if (!whole) {
-                    *reinterpret_cast<float4 *>(piece + row * TN + col) = make_float4(v[0], v[1], v[2], v[3]);
-                } else if (m0 + row < M && n0 + col < N) {
-                    T *c = C + (int64_t)(m0 + row) * ldc + n0 + col;
+                const float w[4] = {o.x, o.y, o.z, o.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) v[e] = acc[i / 2][i % 2 * 4 + e] + w[e];
+            };
+            if (kb1 - kb0 < kblocks) {
+                float *piece = g.ws + ((int64_t)p * 2 + (b == b0 ? 0 : 1)) * (TM * TN) + mrow * TN + ncol;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    float v[4];
+                    sums(i, v);
+                    *reinterpret_cast<float4 *>(piece + i / 2 * TN + i % 2 * 32) = make_float4(v[0], v[1], v[2], v[3]);
+                }
+            } else {
+                // out of the record: the stores below might alias it (read and tested anew for every result, the activation and
+                // the edges made the stores of a tile 16 us)
+                const int M = g.M, N = g.N, act = g.act, vec = g.vec_c;
+                const int64_t ldc = g.ldc;
+                T *C = reinterpret_cast<T *>(g.C) + bn * g.c_stride_n + bc * g.c_stride_c;
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                    const int row = m0 + mrow + i / 2, col = n0 + ncol + i % 2 * 32;
+                    if (row >= M || col >= N) continue;
+                    float v[4];
+                    sums(i, v);
+                    T *c = C + (int64_t)row * ldc + col;
                     if (act != ACT_NONE) {
 #pragma unroll
                         for (int e = 0; e < 4; ++e) v[e] = apply_act(act, v[e]);
                     }
-                    if (vec && n0 + col + 4 <= N) {
+                    if (vec && col + 4 <= N) {
                         store_vec<T, 4>(c, v);
                     } else {
 #pragma unroll
                         for (int e = 0; e < 4; ++e)
-                            if (n0 + col + e < N) c[e] = from_f32<T>(v[e]);
+                            if (col + e < N) c[e] = from_f32<T>(v[e]);
                     }
                 }
             }
@@ -214,9 +224,10 @@ __device__ __noinline__ void simt_sums(const GemmSimtArgs &g, int p, int P) {
 }
 
 // Small products: whole 64 x 64 tiles, 2 x 4 results per thread. A tile is a quarter of the other form's, so that few tiles
-// spread over more CTAs, and costs little besides its multiply-adds; see the rule in the lowering.
+// spread over more CTAs, and costs little besides its multiply-adds; see the rule in the lowering. Not inlined: the registers
+// that the caller would save for it cost the large tiles' stages 4 us each.
 template <typename T>
-__device__ __forceinline__ void simt_small(const GemmSimtArgs &g, int p, int P, float *smem) {
+__device__ __noinline__ void simt_small(const GemmSimtArgs &g, int p, int P, float *smem) {
     constexpr int TM = 64, TN = 64, TK = 16;
     float(*sA)[TM + 1] = reinterpret_cast<float(*)[TM + 1]>(smem);                   // [TK][TM + 1]
     float(*sB)[TN + 1] = reinterpret_cast<float(*)[TN + 1]>(smem + TK * (TM + 1));   // [TK][TN + 1]

@@ -309,9 +309,6 @@ __device__ __noinline__ void gemm_epilogue_tile_partial_rows(const GemmLocal &g,
 //   credited to the leader's `full` barrier; the leader's commits release the
 //   `empty` slot and publish `acc_full` in both CTAs; the epilogue warps of
 //   both CTAs arrive on the leader's `acc_empty`.
-// Warps per accumulator quarter in the epilogue.
-__device__ __forceinline__ int gemm_epi_groups(int tile_n) { return tile_n > 32 ? 2 : 1; }
-
 // Everything the warp roles of one matmul stage share. Built by every thread at the start of the stage; the roles
 // are separate functions (own register allocation: the threads that issue the copies and the MMAs are the critical
 // path of large matmuls, and spills or extra instructions there cost several per cent).
@@ -530,13 +527,12 @@ __device__ __noinline__ bool gemm_issue(const GemmRun &R) {
     return true;
 }
 
-// Epilogue: warps 0-3, each on its 32-lane quarter of the accumulator; with tiles of more than 32 columns also warps 8-11,
-// which take every other block of 32 columns of the same quarters: with four warps a tile's epilogue was about 9 us, which
-// bounds products with a short K and shows after the last tile of any (2048 x 11008 x 4096 with SiLU 188 -> 156 us; the
-// 128-token feed-forward block 63.8 -> 61.7 us; whole sectors per store, see gemm_store16, are part of both).
+// Epilogue: warps 0-3, each on its 32-lane quarter of the accumulator; with two warps per quarter (see the rule in the
+// lowering) also warps 8-11, which take every other block of 32 columns of the same quarters: a 256-column tile's
+// epilogue takes four warps about 9 us.
 template <bool PAIR>
 __device__ __noinline__ bool gemm_drain(const GemmRun &R, int warp_id, int lane) {
-    const int warp = warp_id & 3, grp = warp_id >> 3, grps = gemm_epi_groups(R.L.tile_n);
+    const int warp = warp_id & 3, grp = warp_id >> 3, grps = R.g->epi_groups;
     constexpr bool GROUPED = true;
     const GemmLocal &L = R.L;
     const GemmArgs &g = *R.g;
@@ -695,17 +691,17 @@ __device__ __noinline__ void run_gemm_t(const GemmArgs &g, const GemmArgs *gmaps
     __syncthreads();
 }
 
-// Warps without a role in the matmul (7 and 12..15, with narrow tiles 7..15) do not enter the stage function: its register save area and the
+// Warps without a role in the matmul (7 and 12..15, with one epilogue warp per quarter 7..15) do not enter the stage function: its register save area and the
 // GemmRun record are ~0.5 KB of local memory per thread, and with 208 KiB of the SM's memory configured as shared
 // there is little L1 left to hold them (an idle pass through the function measured 5.5 us). They only take part in
 // the function's three CTA-wide barriers (and the cluster barrier of a pair).
-__device__ __forceinline__ bool gemm_warp_has_role(int tile_n) {
+__device__ __forceinline__ bool gemm_warp_has_role(int epi_groups) {
     const int warp = threadIdx.x >> 5;
-    return warp < kEpiWarps || (gemm_epi_groups(tile_n) == 2 && warp >= 8 && warp < 8 + kEpiWarps) || warp == kProducerWarp || warp == kMmaWarp || warp == kProducerWarpB;
+    return warp < kEpiWarps || (epi_groups == 2 && warp >= 8 && warp < 8 + kEpiWarps) || warp == kProducerWarp || warp == kMmaWarp || warp == kProducerWarpB;
 }
 __device__ __noinline__ void run_gemm(const GemmArgs &g, const GemmArgs *gmaps, int p, int P, char *smem, GemmPipe *pp, CtaCtl *ctl,
                          DeviceState *st, int stage_idx, unsigned long long spin_limit) {
-    if (!gemm_warp_has_role(g.tile_n)) {
+    if (!gemm_warp_has_role(g.epi_groups)) {
         __syncthreads();
         __syncthreads();
         __syncthreads();
@@ -716,7 +712,7 @@ __device__ __noinline__ void run_gemm(const GemmArgs &g, const GemmArgs *gmaps, 
 }
 __device__ __noinline__ void run_gemm_pair(const GemmArgs &g, const GemmArgs *gmaps, int p, int P, char *smem, GemmPipe *pp, CtaCtl *ctl,
                               DeviceState *st, int stage_idx, unsigned long long spin_limit) {
-    if (!gemm_warp_has_role(g.tile_n)) {
+    if (!gemm_warp_has_role(g.epi_groups)) {
         __syncthreads();
         __syncthreads();
         cluster_sync_all();

@@ -726,6 +726,29 @@ struct Lowerer {
         g.vec_c = vec(g.C, g.ldc, g.c_stride_c, g.c_stride_n);
     }
 
+    // Warps per accumulator quarter in the epilogue. Every further warp enters the stage function with its register save area
+    // (1 to 2 us a stage, 5 % of a 4096 x 8192 x 2048 product), so a second one is for epilogues that cost more than that.
+    // One B200, fp16, M x N x K, us with one and two warps:
+    //  * activations: gelu 2048 x 4096 x 1024 84 and 56, 300 x 4096 x 1024 32 and 26, relu 28 and 23;
+    //  * swapped operands, whose results are stored element by element: 64 x 11008 x 4096 57 and 52;
+    //  * accumulators that go out through shared memory and TMA, several tiles per CTA: 4096 x 8192 x 8192 in pairs 410 and
+    //    404, 1080 x 8192 x 8192 in one-CTA tiles 125 and 119 (one tile per CTA, 2048 x 4096 x 8192: 107 and 109);
+    //  * another operand, in pairs, few tiles per pair: 2048 x 4096 x 1024 36 and 34 (five tiles, 2048 x 11008 x 4096: 142 and
+    //    144; one-CTA tiles, 2048 x 4096 x 4096: 67 and 70);
+    //  * rows stored as they are, several tiles per CTA and a short K: 4096 x 8192 by 256, 512, 1024, 2048 56 and 52, 60 and
+    //    57, 69 and 70, 104 and 111;
+    //  * not fp32 partials of ordinary tiles: 512 x 1024 x 4096 31 and 33.
+    int32_t epilogue_groups(const Stage &s) const {
+        const GemmArgs &g = s.gm;
+        if (g.tile_n <= 32) return 1;
+        if (g.out_transposed) return 2;
+        if (g.splits > 1) return 1;
+        if (g.act != ACT_NONE) return 2;
+        const int64_t ctas = (s.proc_e - s.proc_b + s.proc_s - 1) / s.proc_s, at_once = prog.pair_mode ? ctas / 2 : ctas;
+        if (g.bias) return prog.pair_mode && g.n_units <= 2 * at_once ? 2 : 1;
+        return g.n_units > at_once && (g.c_tma || g.K <= 512) ? 2 : 1;
+    }
+
     void lower_matmul(const OpDesc &op, const Range &proc, const TaskGroup &tg, int act, const TensorDesc *act_out,
                       const OpDesc *fuse_ar = nullptr, const GemvFuse *gf = nullptr, const TensorDesc *epi = nullptr,
                       int epi_mode = 0 /* 0: add, 1: multiply, 2: rotary table [rope_rows][rope_cols] */, int64_t rope_rows = 0,
@@ -2853,6 +2876,12 @@ struct Lowerer {
         elide_syncs();
         pair_weight_streams();
         plan_prefetch();
+        for (size_t i = 0; i < prog.stages.size(); ++i) {
+            Stage &s = prog.stages[i];
+            if (s.kind != SK_GEMM) continue;
+            s.gm.epi_groups = epilogue_groups(s);
+            if (s.gm.epi_groups == 2) prog.notes[i] += " epilogue=8 warps";
+        }
         // dynamic shared memory: the largest need of any stage
         auto need_of = [](const Stage &s) {
             size_t need = 0;

@@ -210,7 +210,7 @@ struct GemmArgs {
                                      // halves take both accumulator buffers, so the epilogue does not overlap the next tile
     float *ws;                       // split-K partials, layout [splits][batch][rows of C][cols of C]
     int32_t peer_rows;               // > 0: fused all_reduce, rows of C each rank sums (M / ranks)
-    int32_t pad3;
+    int32_t epi_groups;              // warps per accumulator quarter in the epilogue: 1 or 2
 };
 
 // Second half of a split-K matmul: C = act(sum_s ws[s] + bias), one rounding.

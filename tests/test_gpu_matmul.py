@@ -60,6 +60,22 @@ def test_matmul_fused_activation(fuse):
     assert_matmul_close(got, want, "fp16", f"fused {fuse}")
 
 
+@pytest.mark.parametrize("mnk,ta,tb,act,eight", [
+    ((300, 1000, 1024), False, True, None, False),    # rows stored as they are
+    ((1100, 4104, 264), False, True, None, True),     # several tiles per CTA, short K
+    ((1100, 4104, 1032), False, False, None, False),
+    ((260, 4104, 1024), False, True, "gelu", True),   # an activation
+    ((520, 8200, 8192), False, True, None, True),     # through shared memory, several tiles per CTA
+    ((1030, 3080, 8192), False, True, None, False),   # one
+])
+def test_matmul_epilogue_on_four_and_eight_warps(mnk, ta, tb, act, eight):
+    from ark_b200.executor import plan_dump
+    m, n, k = mnk
+    got, want = run_mm((k, m) if ta else (m, k), (n, k) if tb else (k, n), "fp16", ta, tb, fuse=act)
+    assert ("epilogue=8 warps" in plan_dump(str(ark.Planner(0).plan()))) == eight
+    assert_matmul_close(got, want, "fp16", f"epilogue {mnk}")
+
+
 def test_matmul_constant_inputs():
     # ops_matmul_test.cpp:343-360: all 0.1 -> every output is k * 0.01
     ark.init()

@@ -628,6 +628,21 @@ def test_small_full_precision_products_take_small_tiles(a, b, small):
     assert ("tile=64x64" in text) == small, text
 
 
+@pytest.mark.parametrize("m,n,k,act,eight", [
+    (128, 8192, 8192, False, False), (512, 1024, 4096, False, False),                                     # split-K partials
+    (2048, 4096, 4096, False, False), (2048, 4096, 4096, True, True), (4096, 8192, 2048, False, False),   # rows, activations
+    (4096, 8192, 512, False, True), (2048, 2048, 512, False, False), (64, 11008, 4096, False, True),      # short K, swapped
+    (4096, 8192, 8192, False, True), (128, 4096, 1024, True, False),                                      # TMA, narrow tiles
+])
+def test_epilogue_takes_eight_warps_where_that_is_faster(m, n, k, act, eight):
+    def build():
+        with ark.PlannerContext(sync=False):
+            y = ark.matmul(ark.tensor([m, k], ark.fp16), ark.tensor([n, k], ark.fp16), transpose_other=True)
+            return ark.gelu(y) if act else y
+    text = _stages(build)
+    assert ("epilogue=8 warps" in text) == eight, text
+
+
 def test_ring_of_few_rows_is_short_only_where_the_plan_stays_small():
     """Three slots next to stages that need as little shared memory, six (a pair of CTAs shares the activations) next to one
     that takes all of it."""

@@ -729,7 +729,7 @@ __device__ __noinline__ void run_gemm_pair(const GemmArgs &g, const GemmArgs *gm
 // warps without a share do not enter (16 warps' register saves were 4 us of a 7 us stage).
 template <typename T>
 __device__ __noinline__ void splitk_reduce_typed(const SplitKReduceArgs &a, int p, int P) {
-    const int64_t per = (int64_t)a.M * a.N, total = per * a.batch_c * a.batch_n;
+    const int64_t total = (int64_t)a.M * a.N * a.batch_c * a.batch_n;
     const int64_t tid = ((int64_t)(threadIdx.x >> 5) * P + p) * 32 + (threadIdx.x & 31), nth = (int64_t)P * kThreads;
     const bool vec = (a.N % 4 == 0);
     const int64_t step = vec ? 4 : 1;
@@ -751,14 +751,36 @@ __device__ __noinline__ void splitk_reduce_typed(const SplitKReduceArgs &a, int 
         } else {
             for (int s = 0; s < splits; ++s) acc[0] += a.ws[(int64_t)s * total + e0];
         }
-        for (int i = 0; i < step; ++i) {
-            const int64_t e = e0 + i;
-            const int64_t b = e / per, r = e % per;
-            const int64_t m = r / a.N, n = r % a.N;
-            const int64_t off = (b / a.batch_c) * a.c_stride_n + (b % a.batch_c) * a.c_stride_c + m * a.ldc + n;
-            float v = acc[i];
-            if (a.bias) v += to_f32(reinterpret_cast<const T *>(a.bias)[off]);
-            reinterpret_cast<T *>(a.C)[off] = from_f32<T>(apply_act_fast(a.act, v));
+        // the results of a step are neighbours in a row
+        int64_t off;
+        if (total <= UINT32_MAX) {  // 64-bit divisions for every element were a fifth of the stage
+            const uint32_t row = (uint32_t)e0 / (uint32_t)a.N, b = row / (uint32_t)a.M;
+            off = (int64_t)(b / a.batch_c) * a.c_stride_n + (int64_t)(b % a.batch_c) * a.c_stride_c + (int64_t)(row - b * a.M) * a.ldc + ((uint32_t)e0 - row * a.N);
+        } else {
+            const int64_t row = e0 / a.N, b = row / a.M;
+            off = (b / a.batch_c) * a.c_stride_n + (b % a.batch_c) * a.c_stride_c + (row - b * a.M) * a.ldc + (e0 - row * a.N);
+        }
+        T *c = reinterpret_cast<T *>(a.C) + off;
+        const T *bias = a.bias ? reinterpret_cast<const T *>(a.bias) + off : nullptr;
+        if (vec && ((reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(bias)) & (4 * sizeof(T) - 1)) == 0) {
+            if (bias) {
+                float f[4];
+                load_vec<T, 4>(bias, f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] += f[i];
+            }
+            if (a.act != ACT_NONE) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[i] = apply_act_fast(a.act, acc[i]);
+            }
+            store_vec<T, 4>(c, acc);
+        } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                if (i >= step) break;
+                if (bias) acc[i] += to_f32(bias[i]);
+                c[i] = from_f32<T>(apply_act_fast(a.act, acc[i]));
+            }
         }
     }
 }

@@ -370,6 +370,29 @@ def test_matmul_few_long_tiles_split_k(dt, mnk, tb, fuse):
     assert_matmul_close(got, want, dt, f"split-K tiles {mnk}")
 
 
+@pytest.mark.parametrize("m,n,k,pitch", [(40, 1024, 4096, 1024), (40, 1024, 4096, 1026), (40, 1024, 4096, 1028), (40, 1020, 4096, 1020),
+                                         (40, 1023, 4096, 1032), (1024, 124, 8192, 0)])
+def test_split_k_sum_stores(m, n, k, pitch):
+    """Rows of whole, half and no 8-byte vectors of results; without a pitch, another operand is added."""
+    rng = np.random.default_rng(37)
+    a, b, r = rand(rng, (m, k), "bf16"), O.to_storage(rng.normal(0, 0.05, (n, k)).astype(np.float32), "bf16"), rand(rng, (m, n), "bf16")
+    ark.init()
+    t_a, t_b, t_r = ark.tensor([m, k], ark.bf16), ark.tensor([n, k], ark.bf16), ark.tensor([m, n], ark.bf16)
+    feeds = {t_a: a, t_b: b}
+    with ark.PlannerContext(sync=False):
+        if pitch:
+            y = ark.matmul(t_a, t_b, transpose_other=True, output=ark.tensor([m, n], ark.bf16, strides=[m, pitch], padded_shape=[m, n]))
+        else:
+            y = ark.add(ark.matmul(t_a, t_b, transpose_other=True), t_r)
+            feeds[t_r] = r
+    text = ark.plan_dump(str(ark.Planner(0).plan()))
+    assert "split-K sum" in text and " Add " not in text, text
+    (got,) = execute([y], feeds)
+    want = O.matmul(O.to_f32(a, "bf16"), O.to_f32(b, "bf16"), "fp32", False, True)
+    want = O.to_storage(want if pitch else O.binary("add", want, O.to_f32(r, "bf16"), "fp32"), "bf16")
+    assert_matmul_close(got, want, "bf16", f"split-K sum {n} {pitch}")
+
+
 def test_matmul_split_k_tiles_are_chosen():
     """The lowering cuts K only where the model says it pays (a [4096, 128] output over K = 8192), and an Add folded into
     the epilogue moves to the sum stage."""

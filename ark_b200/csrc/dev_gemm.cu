@@ -1,4 +1,4 @@
-// Tile loops of the tensor-core matmul and the CUDA-core fallback (see dev_gemm.cuh).
+// Tile loops of the tensor-core matmul and the sums of its split-K partials (see dev_gemm.cuh).
 #include "dev_gemm.cuh"
 
 namespace arkb {
@@ -77,16 +77,18 @@ __device__ __forceinline__ void gemm_load16(const T *p, float (&f)[16], bool wid
     for (int i = 0; i < 16; ++i) f[i] = to_f32(o.e[i]);
 }
 
-template <typename T>
+// OPERAND: with another operand (brow) or a rotary table.
+template <typename T, bool OPERAND>
 __device__ __forceinline__ void gemm_store_row(const GemmLocal &g, T *crow, const T *brow, int col, int ncols,
                                                uint32_t (&r)[32], int cnt, int bcol0 = 0) {
+    if constexpr (!OPERAND) brow = nullptr;
     // cnt accumulator values (16 or 32) for columns [col, col+cnt) of one row
     float f[32];
 #pragma unroll
     for (int i = 0; i < 32; ++i) f[i] = (i < cnt) ? __uint_as_float(r[i]) : 0.0f;
     const bool full = (col + cnt <= ncols) && g.c_vec;
     const bool wide = (reinterpret_cast<uintptr_t>(crow + col) & 31) == 0;
-    if (g.bias_mul == 2) {
+    if (OPERAND && g.bias_mul == 2) {
         // rotary embedding on the accumulator: brow is the table row of this output row, bcol0 the absolute column of
         // column 0 of `crow` (even; the table row length is a multiple of 8, so an 8-vector never wraps)
 #pragma unroll
@@ -182,14 +184,16 @@ __device__ __noinline__ void gemm_epilogue_tile_tma(const GemmLocal &g, const CU
     }
 }
 
-template <typename T>
+// Two functions, so that the plain one does not save registers for the operand (half a microsecond a stage: 128 x 4096 x 1024
+// 15.5 us with one function for both).
+template <typename T, bool OPERAND>
 __device__ __noinline__ void gemm_epilogue_tile(const GemmLocal &g, const TileCoord &tc, uint32_t tmem_acc, int warp, int lane, int grp, int grps) {
     const int row = tc.m0 + warp * 32 + lane;
     const bool row_ok = row < g.M;
     const int64_t boff = (int64_t)tc.bn * g.c_stride_n + (int64_t)tc.bc * g.c_stride_c + (int64_t)row * g.ldc;
     T *crow = reinterpret_cast<T *>(g.C) + boff;
-    const T *brow = g.bias ? reinterpret_cast<const T *>(g.bias) + boff : nullptr;
-    if (g.bias_mul == 2) brow = reinterpret_cast<const T *>(g.bias) + (int64_t)(row_ok ? row % g.rope_rows : 0) * g.rope_cols - tc.n0;
+    const T *brow = OPERAND ? reinterpret_cast<const T *>(g.bias) + boff : nullptr;
+    if (OPERAND && g.bias_mul == 2) brow = reinterpret_cast<const T *>(g.bias) + (int64_t)(row_ok ? row % g.rope_rows : 0) * g.rope_cols - tc.n0;
     const uint32_t lane_addr = tmem_acc + ((uint32_t)(warp * 32) << 16);
     const int ncols_tile = min(g.tile_n, g.N - tc.n0);  // valid columns of this tile
     for (int c = grp * 32; c < g.tile_n; c += grps * 32) {
@@ -199,7 +203,7 @@ __device__ __noinline__ void gemm_epilogue_tile(const GemmLocal &g, const TileCo
         if (cnt == 32) tmem_ld32(lane_addr + c, r);
         else tmem_ld16(lane_addr + c, r);
         tmem_ld_wait();
-        if (row_ok) gemm_store_row<T>(g, crow + tc.n0, brow ? brow + tc.n0 : nullptr, c, ncols_tile, r, cnt, tc.n0);
+        if (row_ok) gemm_store_row<T, OPERAND>(g, crow + tc.n0, OPERAND ? brow + tc.n0 : nullptr, c, ncols_tile, r, cnt, tc.n0);
     }
 }
 
@@ -589,8 +593,13 @@ __device__ __noinline__ bool gemm_drain(const GemmRun &R, int warp_id, int lane)
             if (L.dtype == DT_BF16) gemm_epilogue_tile_tma<__nv_bfloat16>(L, tm, tc, tmem_acc, warp, lane, epi_stage, epi_blk, grp, grps, shift);
             else gemm_epilogue_tile_tma<__half>(L, tm, tc, tmem_acc, warp, lane, epi_stage, epi_blk, grp, grps, shift);
         } else {
-            if (L.dtype == DT_BF16) gemm_epilogue_tile<__nv_bfloat16>(L, tc, tmem_acc, warp, lane, grp, grps);
-            else gemm_epilogue_tile<__half>(L, tc, tmem_acc, warp, lane, grp, grps);
+            auto rows = [&](auto type) {
+                using T = decltype(type);
+                if (L.bias) gemm_epilogue_tile<T, true>(L, tc, tmem_acc, warp, lane, grp, grps);
+                else gemm_epilogue_tile<T, false>(L, tc, tmem_acc, warp, lane, grp, grps);
+            };
+            if (L.dtype == DT_BF16) rows(__nv_bfloat16());
+            else rows(__half());
         }
         tc_fence_before();
         __syncwarp();

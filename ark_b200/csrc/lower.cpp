@@ -727,17 +727,17 @@ struct Lowerer {
     }
 
     // Warps per accumulator quarter in the epilogue. Every further warp enters the stage function with its register save area
-    // (1 to 2 us a stage, 5 % of a 4096 x 8192 x 2048 product), so a second one is for epilogues that cost more than that.
+    // (0.5 to 2 us a stage, 3 % of a 4096 x 8192 x 2048 product), so a second one is for epilogues that cost more than that.
     // One B200, fp16, M x N x K, us with one and two warps:
-    //  * activations: gelu 2048 x 4096 x 1024 84 and 56, 300 x 4096 x 1024 32 and 26, relu 28 and 23;
-    //  * swapped operands, whose results are stored element by element: 64 x 11008 x 4096 57 and 52;
+    //  * activations: gelu 2048 x 4096 x 1024 80 and 51, 300 x 4096 x 1024 31 and 24, relu 26 and 22;
+    //  * swapped operands, whose results are stored element by element: 64 x 11008 x 4096 51 and 46;
     //  * accumulators that go out through shared memory and TMA, several tiles per CTA: 4096 x 8192 x 8192 in pairs 410 and
-    //    404, 1080 x 8192 x 8192 in one-CTA tiles 125 and 119 (one tile per CTA, 2048 x 4096 x 8192: 107 and 109);
-    //  * another operand, in pairs, few tiles per pair: 2048 x 4096 x 1024 36 and 34 (five tiles, 2048 x 11008 x 4096: 142 and
-    //    144; one-CTA tiles, 2048 x 4096 x 4096: 67 and 70);
-    //  * rows stored as they are, several tiles per CTA and a short K: 4096 x 8192 by 256, 512, 1024, 2048 56 and 52, 60 and
-    //    57, 69 and 70, 104 and 111;
-    //  * not fp32 partials of ordinary tiles: 512 x 1024 x 4096 31 and 33.
+    //    403, 1080 x 8192 x 8192 in one-CTA tiles 125 and 119 (one tile per CTA, 2048 x 4096 x 8192: 105 and 106);
+    //  * another operand, in pairs, few tiles per pair: 2048 x 4096 x 1024 36 and 33 (five tiles, 2048 x 11008 x 4096: 142 and
+    //    143; one-CTA tiles, 2048 x 4096 x 4096: 66 and 69);
+    //  * rows stored as they are, several tiles per CTA and a short K: 4096 x 8192 by 256, 512, 1024, 2048 48 and 44, 52 and
+    //    49, 63 and 64, 100 and 104;
+    //  * not fp32 partials of ordinary tiles: 512 x 1024 x 4096 28 and 30.
     int32_t epilogue_groups(const Stage &s) const {
         const GemmArgs &g = s.gm;
         if (g.tile_n <= 32) return 1;
